@@ -20,6 +20,7 @@
 
 #include "internal.cuh"
 #include "plan.h"
+#include "zzx.cuh"
 
 namespace qgpu {
 
@@ -30,13 +31,6 @@ int ff_layout_on(qgpu_handle* h, void* buffer, bool to_pairs);                  
 PlanOptions plan_options_for(const qgpu_handle* h);
 
 constexpr int ADJ_THREADS = 256;
-constexpr int MAX_HAM_QUBITS = 40;
-
-struct Ham {
-    int n;
-    double a[MAX_HAM_QUBITS];
-    double b[MAX_HAM_QUBITS];
-};
 
 // lambda = H psi, and per-block partial sums of Re(conj(psi) lambda). T = double2 (complex128,
 // f64 arithmetic) or float2 (complex64: lambda in f32, the energy sums in f64).
@@ -788,9 +782,14 @@ static int adjoint_sweep_c64(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, c
     float2* lam = (float2*)((uint8_t*)h->work2.ptr + vec);
     double* partial = (double*)((uint8_t*)h->work2.ptr + 2 * vec);
     double* gsum = partial + (nrow_cap + 1) * (size_t)nb;
-    QGPU_CUDA(cudaMemcpyAsync(phi, h->state, vec, cudaMemcpyDeviceToDevice, h->stream));
-    st = energy_into(h, (const float2*)phi, lam, H, partial + nrow_cap * (size_t)nb, energy);
+    bool have = false;
+    if (zzx_tiled_supported(h, H)) st = zzx_tiled(h, h->state, phi, lam, H, energy, &have);
     if (st != QGPU_OK) return st;
+    if (!have) {
+        QGPU_CUDA(cudaMemcpyAsync(phi, h->state, vec, cudaMemcpyDeviceToDevice, h->stream));
+        st = energy_into(h, (const float2*)phi, lam, H, partial + nrow_cap * (size_t)nb, energy);
+        if (st != QGPU_OK) return st;
+    }
     std::vector<std::vector<std::pair<int, double>>> terms(n_ops);
     int nrows = 0;
     std::vector<qgpu_op> seg;  // consecutive multi-wire gates, undone together
@@ -923,6 +922,11 @@ int qgpu_expectation_zzx(qgpu_handle* h, const double* a, const double* b, doubl
     Ham H;
     int st = ham_from(h, a, b, &H);
     if (st != QGPU_OK) return st;
+    if (zzx_tiled_supported(h, H)) {
+        bool ok = false;
+        st = zzx_tiled(h, h->state, nullptr, nullptr, H, energy, &ok);
+        if (st != QGPU_OK || ok) return st;
+    }
     const int nb = adj_blocks(h, h->dim);
     const size_t vec = h->dim * h->amp_bytes;
     st = h->work2.ensure(vec + (size_t)(nb + 8) * 8 + 256);
@@ -978,13 +982,18 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
     double2* lam = (double2*)((uint8_t*)h->work2.ptr + vec);
     double* partial = (double*)((uint8_t*)h->work2.ptr + 2 * vec);
     double* gsum = partial + (nrow_cap + 1) * (size_t)nb;
-    QGPU_CUDA(cudaMemcpyAsync(phi, h->state, vec, cudaMemcpyDeviceToDevice, h->stream));
-    st = energy_into(h, phi, lam, H, partial + nrow_cap * (size_t)nb, energy);
-    if (st != QGPU_OK) return st;
-    // QGPU_MODE_FAST: the sweep works on phi and lambda in the resident float-pair layout (one
-    // conversion each here; the vectors are scratch, nothing converts them back)
+    // QGPU_MODE_FAST: the sweep works on phi and lambda in the resident float-pair layout (the
+    // vectors are scratch, nothing converts them back); the tiled kernels write it directly
     const bool tiles = h->mode == QGPU_MODE_FAST;
-    if (tiles) {
+    bool have = false;
+    if (zzx_tiled_supported(h, H)) st = zzx_tiled(h, h->state, phi, lam, H, energy, &have);
+    if (st != QGPU_OK) return st;
+    if (!have) {
+        QGPU_CUDA(cudaMemcpyAsync(phi, h->state, vec, cudaMemcpyDeviceToDevice, h->stream));
+        st = energy_into(h, phi, lam, H, partial + nrow_cap * (size_t)nb, energy);
+        if (st != QGPU_OK) return st;
+    }
+    if (tiles && !have) {
         st = ff_layout_on(h, phi, true);
         if (st == QGPU_OK) st = ff_layout_on(h, lam, true);
         if (st != QGPU_OK) return st;

@@ -1,0 +1,366 @@
+// zzx.cu — tiled H psi and energy of the ZZ + X observable (no counterpart in quantr).
+//
+// (H psi)[x] = d(x) psi[x] + sum_b c_b psi[x ^ 2^b] needs the n neighbours of every amplitude. The
+// plain kernel (k_apply_zzx, adjoint.cu) gathers them from global memory with f64 arithmetic:
+// n reads through L2 and ~3n operations on the FP64 pipe (1/64 of the FP32 rate) per amplitude.
+// Here a pass takes the neighbours along the bits of a tile of 2^11 amplitudes held in shared
+// memory: the first pass along the 11 lowest bits (and the diagonal), each further pass along 8
+// higher bits (tile: 3 low bits, so that 128-byte runs load together, and the 8 bits), so an n-qubit
+// vector is read 1 + ceil((n - 11) / 8) times. complex128 runs in float pairs (packed Dot2), the
+// energy sum included; complex64 in f32 with the energy as error-free transformed products.
+// What bounds it: the float-pair multiply-adds (12 packed operations per amplitude and bit, ~2.1
+// cycles per amplitude and SM in an 11-bit pass, against 0.7 cycles for its HBM read); complex64:
+// the shared-memory reads (8 of 11 neighbours, 64 B per amplitude) and HBM.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include <math_constants.h>
+
+#include "internal.cuh"
+#include "zzx.cuh"
+
+namespace qgpu {
+
+constexpr int ZZX_THREADS = 256;
+constexpr int ZZX_BITS = 11;    // tile bits: 8 in the thread index, 3 in a thread's registers
+constexpr int ZZX_LOW = 3;      // low bits of the tiles of the later passes
+constexpr int ZZX_REGS = 8;     // amplitudes per thread
+constexpr int ZZX_FIELD = ZZX_BITS - ZZX_LOW;
+
+// Coefficients as the packed operands of a Dot2 term (hi, lo, -hi, -lo), both lanes alike.
+struct ZzxCoef {
+    u64 c[4];
+};
+struct ZzxParams {
+    uint64_t ntiles;
+    int shift;                  // first bit of the tile's high field (later passes)
+    unsigned terms;             // tile bits whose X term this pass adds
+    int n;
+    ZzxCoef x[ZZX_BITS];        // X coefficient of tile bit m
+    // the diagonal (first pass): ZZ coefficient of bits (q, q+1) and of the wrap (0, n-1)
+    float2 zz[MAX_HAM_QUBITS];
+    float2 wrap;
+};
+
+struct ZvFF {
+    using S = double2;
+    using V = ffp;
+    static __device__ __forceinline__ V split(S a) { return to_ffp(a); }
+    // the split keeps neither magnitudes past the float range nor infinities and NaN
+    static __device__ __forceinline__ bool too_large(S a) {
+        constexpr int most = (1023 + 40) << 20;
+        return (__double2hiint(a.x) & 0x7FFFFFFF) >= most || (__double2hiint(a.y) & 0x7FFFFFFF) >= most;
+    }
+    static __device__ __forceinline__ V get(const S* p) { return ffr_load(*p); }
+    static __device__ __forceinline__ void put(S* p, const V& v) { *p = ffr_store(v); }
+    struct Sum {  // sum of coefficient x amplitude
+        PDot2 d;
+        __device__ __forceinline__ void first(const u64* c, const V& v) { d.first(c, v.h, v.l); }
+        __device__ __forceinline__ void add(const u64* c, const V& v) { d.add(c, v.h, v.l); }
+        __device__ __forceinline__ V result() const {
+            V r;
+            d.result(r.h, r.l);
+            return r;
+        }
+    };
+    static __device__ __forceinline__ void term(PDot2& acc, const V& a, const V& b) {
+        const u64 m = p2(-1.f, -1.f);
+        const u64 c[4] = {a.h, a.l, pmul(a.h, m), pmul(a.l, m)};
+        acc.add(c, b.h, b.l);
+    }
+    static __device__ __forceinline__ V plus(const V& a, const V& b) {
+        const u64 t = padd(a.h, b.h);  // TwoSum of the heads, then the tails
+        const u64 bb = psub(t, a.h);
+        u64 e = padd(psub(a.h, psub(t, bb)), psub(b.h, bb));
+        e = padd(e, padd(a.l, b.l));
+        V r;
+        r.h = padd(t, e);
+        r.l = psub(e, psub(r.h, t));
+        return r;
+    }
+};
+
+struct ZvF32 {
+    using S = float2;
+    using V = u64;
+    static __device__ __forceinline__ V split(S a) { return p2(a.x, a.y); }
+    static __device__ __forceinline__ bool too_large(S) { return false; }  // the norm's sum shows it
+    static __device__ __forceinline__ V get(const S* p) { return split(*p); }
+    static __device__ __forceinline__ void put(S* p, V v) {
+        float2 r;
+        up2(v, r.x, r.y);
+        *p = r;
+    }
+    struct Sum {
+        V s;
+        __device__ __forceinline__ void first(const u64* c, V v) { s = pmul(c[0], v); }
+        __device__ __forceinline__ void add(const u64* c, V v) { s = pfma(c[0], v, s); }
+        __device__ __forceinline__ V result() const { return s; }
+    };
+    // the product's rounding error and the sum's both go to the error sum, as in PDot2::add
+    static __device__ __forceinline__ void term(PDot2& acc, V a, V b) {
+        const u64 p = pmul(a, b);
+        const u64 rn = pfma(pmul(a, p2(-1.f, -1.f)), b, p);
+        const u64 t = padd(acc.s, p);
+        const u64 bb = psub(t, acc.s);
+        const u64 q = padd(psub(acc.s, psub(t, bb)), psub(p, bb));
+        acc.s = t;
+        acc.en = padd(psub(acc.en, q), rn);
+    }
+    static __device__ __forceinline__ V plus(V a, V b) { return padd(a, b); }
+};
+
+// (h, l) + (b.x, b.y) as float pairs
+__device__ __forceinline__ float2 ff_plus(float2 a, float2 b) {
+    const float s = __fadd_rn(a.x, b.x);
+    const float bb = __fsub_rn(s, a.x);
+    float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, bb)), __fsub_rn(b.x, bb));
+    e = __fadd_rn(e, __fadd_rn(a.y, b.y));
+    const float h = __fadd_rn(s, e);
+    return make_float2(h, __fsub_rn(e, __fsub_rn(h, s)));
+}
+__device__ __forceinline__ float2 ff_sign(float2 a, unsigned negative) {
+    return negative & 1u ? make_float2(-a.x, -a.y) : a;
+}
+
+__device__ __forceinline__ double zzx_value(const PDot2& acc) {
+    u64 h, l;
+    acc.result(h, l);
+    float h0, h1, l0, l1;
+    up2(h, h0, h1);
+    up2(l, l0, l1);
+    return ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
+}
+
+// FIRST: the diagonal and the 11 lowest bits; otherwise the bits of p.terms (above the 3 lowest).
+// VEC: psi's copy goes to phi and H psi to lam, both in the sweep's layout (P::put); later
+// passes read phi and add to lam. Without VEC only the energy is formed. partial[blockIdx] gets the
+// pass's share of Re <psi|H psi>, and with FIRST partial[gridDim + blockIdx] that of <psi|psi>.
+template <class P, bool FIRST, bool VEC>
+__global__ void __launch_bounds__(ZZX_THREADS, sizeof(typename P::S) == 8 ? 4 : FIRST && VEC ? 2 : 3)
+k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
+      typename P::S* __restrict__ lam, const __grid_constant__ ZzxParams p,
+      double* __restrict__ partial) {
+    using V = typename P::V;
+    __shared__ __align__(16) V tile[1 << ZZX_BITS];
+    __shared__ float2 t_low[64], t_high[64], t_base[4];
+    const unsigned t = threadIdx.x;
+    if (FIRST) {
+        // the diagonal's part inside the tile: pairs of bits 0..5 and of bits 5..10
+        if (t < 128) {
+            const unsigned x = t & 63u;
+            const int q0 = t < 64 ? 0 : 5;
+            float2 d = make_float2(0.f, 0.f);
+            for (int q = 0; q < 5; ++q) d = ff_plus(d, ff_sign(p.zz[q0 + q], (x >> q) ^ (x >> (q + 1))));
+            (t < 64 ? t_low : t_high)[x] = d;
+        }
+    }
+    bool large = false;
+    PDot2 acc, nrm;
+    acc.s = acc.en = nrm.s = nrm.en = 0;
+    for (uint64_t g = blockIdx.x; g < p.ntiles; g += gridDim.x) {
+        uint64_t base, step;  // amplitude of tile index t + 256 j: base + j * step
+        if (FIRST) {
+            base = (g << ZZX_BITS) + t;
+            step = ZZX_THREADS;
+        } else {
+            const uint64_t mid = g & ((1ull << (p.shift - ZZX_LOW)) - 1ull);
+            const uint64_t top = g >> (p.shift - ZZX_LOW);
+            base = (top << (p.shift + ZZX_FIELD)) | (mid << ZZX_LOW) | (t & ((1u << ZZX_LOW) - 1u)) |
+                   ((uint64_t)(t >> ZZX_LOW) << p.shift);
+            step = 1ull << (p.shift + 8 - ZZX_LOW);
+        }
+        V v[ZZX_REGS];
+        if constexpr (!FIRST && VEC) {
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) v[j] = P::get(phi + base + j * step);
+        } else {
+            typename P::S raw[ZZX_REGS];
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) raw[j] = psi[base + j * step];
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) {
+                v[j] = P::split(raw[j]);
+                if constexpr (FIRST) large = large || P::too_large(raw[j]);
+            }
+        }
+        __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) tile[t + ZZX_THREADS * j] = v[j];
+        if (FIRST && t < 32) {
+            // the diagonal's part above the tile, one lane per pair of bits, and its four
+            // combinations with the pairs (10, 11) and (0, n-1) that reach into the tile
+            const int q = ZZX_BITS + (int)t;
+            float2 d = make_float2(0.f, 0.f);
+            if (q + 1 < p.n) d = ff_sign(p.zz[q], (unsigned)((g >> t) ^ (g >> (t + 1))));
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1) {
+                const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d.x, w),
+                                             __shfl_xor_sync(0xffffffffu, d.y, w));
+                d = ff_plus(d, o);
+            }
+            if (t < 4) {
+                d = ff_plus(d, ff_sign(p.zz[ZZX_BITS - 1], (t & 1u) ^ (unsigned)(g & 1ull)));
+                d = ff_plus(d, ff_sign(p.wrap, (t >> 1) ^ (unsigned)(g >> (p.n - 1 - ZZX_BITS))));
+                t_base[t] = d;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) {
+            typename P::Sum s;
+            if constexpr (FIRST) {
+                float2 d = ff_plus(t_low[t & 63u], t_high[((t >> 5) & 7u) | (j << 3)]);
+                d = ff_plus(d, t_base[(j >> 2) | ((t & 1u) << 1)]);
+                const u64 c[4] = {p2(d.x, d.x), p2(d.y, d.y), p2(-d.x, -d.x), p2(-d.y, -d.y)};
+                s.first(c, v[j]);
+            } else {
+                const u64 zero[4] = {0, 0, 0, 0};
+                s.first(zero, v[j]);
+            }
+#pragma unroll
+            for (int m = FIRST ? 0 : ZZX_LOW; m < 8; ++m)
+                if ((p.terms >> m) & 1u) s.add(p.x[m].c, tile[(t ^ (1u << m)) + ZZX_THREADS * j]);
+#pragma unroll
+            for (int m = 8; m < ZZX_BITS; ++m)
+                if ((p.terms >> m) & 1u) s.add(p.x[m].c, v[j ^ (1 << (m - 8))]);
+            const V o = s.result();
+            P::term(acc, v[j], o);
+            if constexpr (FIRST) P::term(nrm, v[j], v[j]);
+            if constexpr (VEC) {
+                if constexpr (FIRST) {
+                    P::put(phi + base + j * step, v[j]);
+                    P::put(lam + base + j * step, o);
+                } else {
+                    P::put(lam + base + j * step, P::plus(P::get(lam + base + j * step), o));
+                }
+            }
+        }
+    }
+    // per-CTA sums: warp shuffles, then one value per warp
+    double e = zzx_value(acc), q = FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        e += __shfl_down_sync(0xffffffffu, e, w);
+        if (FIRST) q += __shfl_down_sync(0xffffffffu, q, w);
+    }
+    __shared__ double sums[2][ZZX_THREADS / 32];
+    if ((t & 31u) == 0) {
+        sums[0][t >> 5] = e;
+        sums[1][t >> 5] = q;
+    }
+    __syncthreads();
+    if (t < (FIRST ? 2u : 1u)) {
+        double s = 0.0;
+        for (int w = 0; w < ZZX_THREADS / 32; ++w) s += sums[t][w];
+        partial[t * gridDim.x + blockIdx.x] = s;
+    }
+}
+
+// out[r] = sum of row r (nb values each): one warp per row, fixed order
+__global__ void k_zzx_rows(const double* __restrict__ partial, int nb, double* __restrict__ out) {
+    const int row = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int b = lane; b < nb; b += 32) s += partial[(size_t)row * nb + b];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+    if (lane == 0) out[row] = s;
+}
+
+static float2 coef_pair(double c) {
+    const float h = (float)c;
+    return make_float2(h, (float)(c - (double)h));
+}
+static u64 both(float f) {
+    uint32_t b;
+    std::memcpy(&b, &f, 4);
+    return (u64)b | ((u64)b << 32);
+}
+
+template <class P, bool VEC>
+static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
+                   typename P::S* lam, const Ham& H, double* energy, bool* ok) {
+    const int n = H.n;
+    static_assert(1 + (MAX_HAM_QUBITS - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD + 1 <= 8, "row sums");
+    const int npass = 1 + (n - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx<P, true, VEC>, ZZX_THREADS, 0) !=
+            cudaSuccess || occ < 1)
+        occ = 1;
+    const uint64_t ntiles = h->dim >> ZZX_BITS;
+    const int nb = (int)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * occ);
+    int st = h->work.ensure(((size_t)(npass + 1) * nb + npass + 1) * sizeof(double));
+    if (st != QGPU_OK) return st;
+    double* partial = (double*)h->work.ptr;
+    double* sums = partial + (size_t)(npass + 1) * nb;
+    ZzxParams p;
+    std::memset(&p, 0, sizeof(p));
+    p.ntiles = ntiles;
+    p.n = n;
+    for (int q = 0; q + 1 < n; ++q) p.zz[q] = coef_pair(H.a[n - 2 - q]);  // wires n-2-q, n-1-q
+    p.wrap = coef_pair(H.a[n - 1]);
+    int done = 0;  // bits whose X term has been added
+    for (int pass = 0; pass < npass; ++pass) {
+        int first = 0, low = 0;  // tile bit m >= low is index bit first + m - low
+        if (pass > 0) {
+            first = std::min(done, n - ZZX_FIELD);  // the last field may reach back over done bits
+            low = ZZX_LOW;
+            p.shift = first;
+        }
+        p.terms = 0;
+        for (int m = low; m < ZZX_BITS; ++m) {
+            const int bit = first + m - low;
+            if (bit < done || bit >= n) continue;
+            p.terms |= 1u << m;
+            const float2 c = coef_pair(H.b[n - 1 - bit]);
+            p.x[m].c[0] = both(c.x);
+            p.x[m].c[1] = both(c.y);
+            p.x[m].c[2] = both(-c.x);
+            p.x[m].c[3] = both(-c.y);
+        }
+        done = first + ZZX_BITS - low;
+        if (pass == 0)
+            k_zzx<P, true, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, partial);
+        else
+            k_zzx<P, false, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(
+                psi, phi, lam, p, partial + (size_t)(pass + 1) * nb);
+        QGPU_CHECK_LAUNCH("k_zzx");
+        h->launches++;
+        h->h2d_bytes += sizeof(p);
+    }
+    k_zzx_rows<<<1, 32 * (npass + 1), 0, h->stream>>>(partial, nb, sums);
+    QGPU_CHECK_LAUNCH("k_zzx_rows");
+    h->launches++;
+    double host[8];
+    QGPU_CUDA(copy_async(h, host, sums, (npass + 1) * sizeof(double), cudaMemcpyDeviceToHost));
+    QGPU_CUDA(cudaStreamSynchronize(h->stream));
+    *energy = host[0];
+    for (int r = 2; r <= npass; ++r) *energy += host[r];
+    // amplitudes near one scale: their products keep their rounding errors in float range
+    *ok = host[1] > 0x1p-40 && host[1] < 0x1p40;
+    return QGPU_OK;
+}
+
+bool zzx_tiled_supported(const qgpu_handle* h, const Ham& H) {
+    if (h->n_qubits < ZZX_MIN_QUBITS || (h->precision == QGPU_C128 && h->mode != QGPU_MODE_FAST))
+        return false;
+    double most = 0.0;
+    for (int i = 0; i < H.n; ++i) {
+        if (!std::isfinite(H.a[i]) || !std::isfinite(H.b[i])) return false;
+        most = std::max(most, std::max(std::fabs(H.a[i]), std::fabs(H.b[i])));
+    }
+    return most > 0x1p-40 && most < 0x1p40;
+}
+
+int zzx_tiled(qgpu_handle* h, const void* psi, void* phi, void* lam, const Ham& H, double* energy,
+              bool* ok) {
+    if (h->precision == QGPU_C64)
+        return lam ? run_zzx<ZvF32, true>(h, (const float2*)psi, (float2*)phi, (float2*)lam, H, energy, ok)
+                   : run_zzx<ZvF32, false>(h, (const float2*)psi, nullptr, nullptr, H, energy, ok);
+    return lam ? run_zzx<ZvFF, true>(h, (const double2*)psi, (double2*)phi, (double2*)lam, H, energy, ok)
+               : run_zzx<ZvFF, false>(h, (const double2*)psi, nullptr, nullptr, H, energy, ok);
+}
+
+}  // namespace qgpu
