@@ -6,11 +6,11 @@
 // For a rotation U_l = exp(-i theta P / 2) (quantr's Rx, Ry, Rz; P = X, Y, Z) the derivative is
 // dE/dtheta_l = 2 Re <lambda_l| dU_l |psi_{l-1}> = Im <lambda_l| P |phi_l>, read from the two
 // vectors before the gate is undone; Phase(theta) = exp(i theta / 2) I gives -Im <lambda|phi>.
-// Then phi <- U_l^dagger phi and lambda <- U_l^dagger lambda. In QGPU_MODE_FAST the runs of
-// single-wire gates go through k_adj_tile (all gates of a wire, or of two wires, per pass, float-
-// pair arithmetic), or up to 22 qubits k_adj_group (the wires of a tile of up to 11 bits per
-// pass); QGPU_MODE_F64 uses k_adj_1q, one gate per pass in f64. Multi-wire gates are
-// undone with the fused gate passes of program.cu on each vector.
+// Then phi <- U_l^dagger phi and lambda <- U_l^dagger lambda. In QGPU_MODE_FAST and complex64 the
+// runs of single-wire gates go through k_adj_group (adj_group.cu: the wires of a tile of up to 10
+// or 11 bits per pass); with QGPU_ADJ_GROUP=0 the complex128 ones through k_adj_tile (all gates of a
+// wire, or of two wires, per pass). QGPU_MODE_F64 uses k_adj_1q, one gate per pass in f64.
+// Multi-wire gates are undone with the fused gate passes of program.cu on each vector.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -18,6 +18,7 @@
 #include <cstring>
 #include <vector>
 
+#include "adj_group.cuh"
 #include "internal.cuh"
 #include "plan.h"
 #include "zzx.cuh"
@@ -342,175 +343,6 @@ k_adj_tile(double2* __restrict__ phi, double2* __restrict__ lam,
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// k_adj_group: the runs of single-wire gates of the reverse sweep on up to ADJ_GROUP_MAX_BITS
-// wires in one pass over phi and lambda (in place, resident float-pair layout). A CTA stages a
-// tile of both vectors in shared memory: the 2^K amplitudes that share every bit outside the
-// pass's K tile bits (the wires' bits and the lowest other bits, so that 32 consecutive
-// amplitudes load together). Then, wire by wire, each thread takes the wire's Pauli sums over its
-// pairs (packed Dot2, reduced per warp in float pairs into shared accumulators) and applies the
-// run's undo to its pairs of both vectors. Gates on different wires commute and a wire's sums are
-// taken before its own undo, so the results are those of one pass per wire (k_adj_tile with
-// Pauli steps), with one read and one write of each vector per pass.
-// ---------------------------------------------------------------------------------------------
-constexpr int ADJ_GROUP_MAX_BITS = ADJ_GROUP_TILE_BITS;
-constexpr int ADJ_GROUP_THREADS = 256;
-constexpr int ADJ_GROUP_WARPS = ADJ_GROUP_THREADS / 32;
-
-struct AdjGroupWire {
-    int lb;      // tile bit of the wire
-    int row[4];  // partial rows of its sums over X, Y, Z, -I (-1: not needed)
-    u64 pk[32];  // ST_DENSE packed constants of the run's undo
-};
-struct AdjGroupParams {
-    uint64_t ngroups;
-    int nbits;
-    int bits[ADJ_GROUP_MAX_BITS];  // ascending
-    int nwires;
-    int nb;                        // row length of partial (>= the grid)
-    AdjGroupWire w[ADJ_GROUP_MAX_BITS];
-};
-
-__host__ __device__ constexpr size_t adj_group_smem(int nbits) {
-    return (size_t)2 * 16 * ((size_t)1 << nbits) + (size_t)ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4 * 8 +
-           (32 + 64) * 8;
-}
-
-// (h, l) += (bh, bl) in float-pair arithmetic (TwoSum of the heads, then the tails)
-__device__ __forceinline__ void ff2_acc(float& h, float& l, float bh, float bl) {
-    const float s = __fadd_rn(h, bh);
-    const float bb = __fadd_rn(s, -h);
-    float e = __fadd_rn(__fadd_rn(h, -__fadd_rn(s, -bb)), __fadd_rn(bh, -bb));
-    e = __fadd_rn(e, __fadd_rn(l, bl));
-    h = __fadd_rn(s, e);
-    l = __fadd_rn(e, -__fadd_rn(h, -s));
-}
-
-__global__ void __launch_bounds__(ADJ_GROUP_THREADS, 2)
-k_adj_group(double2* __restrict__ phi, double2* __restrict__ lam,
-            const __grid_constant__ AdjGroupParams p, double* __restrict__ partial) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int T = 1 << p.nbits;
-    double2* sf = reinterpret_cast<double2*>(smem);    // phi tile
-    double2* sl = sf + T;                               // lambda tile
-    float2* sacc = reinterpret_cast<float2*>(sl + T);   // [warp][wire][pauli] float pairs
-    uint64_t* lo_tab = reinterpret_cast<uint64_t*>(sacc + ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4);
-    uint64_t* hi_tab = lo_tab + 32;                     // [T >> nlo] (at most 64)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nlo = p.nbits < 5 ? p.nbits : 5;
-    for (int i = tid; i < 32 + (T >> nlo); i += ADJ_GROUP_THREADS) {
-        uint64_t o = 0;
-        if (i < 32) {
-            for (int m = 0; m < nlo; ++m)
-                if ((i >> m) & 1) o |= 1ull << p.bits[m];
-            lo_tab[i] = o;
-        } else {
-            const int v = i - 32;
-            for (int m = nlo; m < p.nbits; ++m)
-                if ((v >> (m - nlo)) & 1) o |= 1ull << p.bits[m];
-            hi_tab[v] = o;
-        }
-    }
-    for (int i = tid; i < ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4; i += ADJ_GROUP_THREADS)
-        sacc[i] = make_float2(0.f, 0.f);
-    __syncthreads();
-    const int lomask = (1 << nlo) - 1;
-    for (uint64_t g = blockIdx.x; g < p.ngroups; g += gridDim.x) {
-        uint64_t base = g;
-        for (int m = 0; m < p.nbits; ++m) base = insert_zero(base, p.bits[m]);
-        for (int i = tid; i < T; i += ADJ_GROUP_THREADS) {
-            const uint64_t o = base | lo_tab[i & lomask] | hi_tab[i >> nlo];
-            sf[i] = phi[o];
-            sl[i] = lam[o];
-        }
-        __syncthreads();
-        for (int w = 0; w < p.nwires; ++w) {
-            const int lb = p.w[w].lb;
-            const u64* pk = p.w[w].pk;
-            PDot2 acc[4];
-            bool first[4] = {true, true, true, true};
-            const bool need[4] = {p.w[w].row[0] >= 0, p.w[w].row[1] >= 0, p.w[w].row[2] >= 0,
-                                  p.w[w].row[3] >= 0};
-            for (int q = tid; q < (T >> 1); q += ADJ_GROUP_THREADS) {
-                const int i0 = ((q >> lb) << (lb + 1)) | (q & ((1 << lb) - 1));
-                const int i1 = i0 | (1 << lb);
-                ffp f0 = ffr_load(sf[i0]), f1 = ffr_load(sf[i1]);
-                ffp l0 = ffr_load(sl[i0]), l1 = ffr_load(sl[i1]);
-                ffp f0s, f1s;  // swapped lanes (im, re)
-                f0s.h = pswap(f0.h);
-                f0s.l = pswap(f0.l);
-                f1s.h = pswap(f1.h);
-                f1s.l = pswap(f1.l);
-                if (need[0]) {  // X: Im(l0* f1) + Im(l1* f0)
-                    adj_term(acc[0], first[0], l0, f1s, 1.f, -1.f);
-                    adj_term(acc[0], first[0], l1, f0s, 1.f, -1.f);
-                }
-                if (need[1]) {  // Y: -Re(l0* f1) + Re(l1* f0)
-                    adj_term(acc[1], first[1], l0, f1, -1.f, -1.f);
-                    adj_term(acc[1], first[1], l1, f0, 1.f, 1.f);
-                }
-                if (need[2]) {  // Z: Im(l0* f0) - Im(l1* f1)
-                    adj_term(acc[2], first[2], l0, f0s, 1.f, -1.f);
-                    adj_term(acc[2], first[2], l1, f1s, -1.f, 1.f);
-                }
-                if (need[3]) {  // global phase: -(Im(l0* f0) + Im(l1* f1))
-                    adj_term(acc[3], first[3], l0, f0s, -1.f, 1.f);
-                    adj_term(acc[3], first[3], l1, f1s, -1.f, 1.f);
-                }
-                ff_dense(f0, f1, pk);
-                ff_dense(l0, l1, pk);
-                sf[i0] = ffr_store(f0);
-                sf[i1] = ffr_store(f1);
-                sl[i0] = ffr_store(l0);
-                sl[i1] = ffr_store(l1);
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                if (!need[m]) continue;
-                float h = 0.f, l = 0.f;
-                if (!first[m]) {
-                    u64 rh, rl;
-                    acc[m].result(rh, rl);
-                    float h1, l1;
-                    up2(rh, h, h1);
-                    up2(rl, l, l1);
-                    ff2_acc(h, l, h1, l1);
-                }
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) {
-                    const float oh = __shfl_down_sync(0xffffffffu, h, d);
-                    const float ol = __shfl_down_sync(0xffffffffu, l, d);
-                    ff2_acc(h, l, oh, ol);
-                }
-                if (lane == 0) {
-                    float2& a = sacc[(warp * ADJ_GROUP_MAX_BITS + w) * 4 + m];
-                    ff2_acc(a.x, a.y, h, l);
-                }
-            }
-            __syncthreads();
-        }
-        for (int i = tid; i < T; i += ADJ_GROUP_THREADS) {
-            const uint64_t o = base | lo_tab[i & lomask] | hi_tab[i >> nlo];
-            phi[o] = sf[i];
-            lam[o] = sl[i];
-        }
-        __syncthreads();
-    }
-    // per-CTA sums into column blockIdx.x; columns past the grid (partial rows have nb columns) get 0
-    for (int k = tid; k < p.nwires * 4; k += ADJ_GROUP_THREADS) {
-        const int w = k >> 2, m = k & 3;
-        if (p.w[w].row[m] < 0) continue;
-        double t = 0.0;
-        for (int v = 0; v < ADJ_GROUP_WARPS; ++v) {
-            const float2 a = sacc[(v * ADJ_GROUP_MAX_BITS + w) * 4 + m];
-            t += (double)a.x + (double)a.y;
-        }
-        double* row = partial + (size_t)p.w[w].row[m] * p.nb;
-        row[blockIdx.x] = t;
-        for (int c = blockIdx.x + gridDim.x; c < p.nb; c += gridDim.x) row[c] = 0.0;
-    }
-}
-
 // Event-timed launch under qgpu_set_profiling (filed under `name`, bytes = reads + writes of both
 // vectors); a plain launch otherwise.
 template <class F>
@@ -528,154 +360,6 @@ static int adj_profiled(qgpu_handle* h, const char* name, double bytes, F&& laun
         return prof_collect(h, {name}, {bytes});
     }
     return QGPU_OK;
-}
-
-static int launch_adj_group(qgpu_handle* h, double2* phi, double2* lam, const AdjGroupParams& p,
-                            double* partial) {
-    const size_t smem = adj_group_smem(p.nbits);
-    QGPU_CUDA(smem_opt_in((const void*)k_adj_group, adj_group_smem(ADJ_GROUP_MAX_BITS)));
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adj_group, ADJ_GROUP_THREADS, smem) != cudaSuccess || occ < 1)
-        occ = 1;
-    const uint64_t grid = std::max<uint64_t>(
-        1, std::min<uint64_t>({p.ngroups, (uint64_t)h->sm_count * occ, (uint64_t)p.nb}));
-    return adj_profiled(h, "k_adj_group", 64.0 * (double)h->dim, [&]() -> int {
-        k_adj_group<<<(unsigned)grid, ADJ_GROUP_THREADS, smem, h->stream>>>(phi, lam, p, partial);
-        QGPU_CHECK_LAUNCH("k_adj_group");
-        h->launches++;
-        h->h2d_bytes += sizeof(p);
-        return QGPU_OK;
-    });
-}
-
-// k_adj_group_f32: k_adj_group for complex64 vectors. Plain f32 complex arithmetic for the Pauli
-// sums and the undo, the sums reduced per warp in f32 and accumulated per CTA in f64.
-struct AdjGroupWireF {
-    int lb;      // tile bit of the wire
-    int row[4];  // partial rows of its sums over X, Y, Z, -I (-1: not needed)
-    float u[8];  // the run's undo, row-major complex (u00, u01, u10, u11)
-};
-struct AdjGroupParamsF {
-    uint64_t ngroups;
-    int nbits;
-    int bits[ADJ_GROUP_MAX_BITS];
-    int nwires;
-    int nb;
-    AdjGroupWireF w[ADJ_GROUP_MAX_BITS];
-};
-
-__host__ __device__ constexpr size_t adj_group_f32_smem(int nbits) {
-    return (size_t)2 * 8 * ((size_t)1 << nbits) + (size_t)ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4 * 8 +
-           (32 + 64) * 8;
-}
-
-__device__ __forceinline__ float2 cmul_add(float ur, float ui, float2 a, float vr, float vi, float2 b) {
-    return make_float2(fmaf(ur, a.x, fmaf(-ui, a.y, fmaf(vr, b.x, -vi * b.y))),
-                       fmaf(ur, a.y, fmaf(ui, a.x, fmaf(vr, b.y, vi * b.x))));
-}
-
-__global__ void __launch_bounds__(ADJ_GROUP_THREADS)
-k_adj_group_f32(float2* __restrict__ phi, float2* __restrict__ lam,
-                const __grid_constant__ AdjGroupParamsF p, double* __restrict__ partial) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int T = 1 << p.nbits;
-    float2* sf = reinterpret_cast<float2*>(smem);
-    float2* sl = sf + T;
-    double* sacc = reinterpret_cast<double*>(sl + T);   // [warp][wire][pauli]
-    uint64_t* lo_tab = reinterpret_cast<uint64_t*>(sacc + ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4);
-    uint64_t* hi_tab = lo_tab + 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nlo = p.nbits < 5 ? p.nbits : 5;
-    for (int i = tid; i < 32 + (T >> nlo); i += ADJ_GROUP_THREADS) {
-        uint64_t o = 0;
-        if (i < 32) {
-            for (int m = 0; m < nlo; ++m)
-                if ((i >> m) & 1) o |= 1ull << p.bits[m];
-            lo_tab[i] = o;
-        } else {
-            const int v = i - 32;
-            for (int m = nlo; m < p.nbits; ++m)
-                if ((v >> (m - nlo)) & 1) o |= 1ull << p.bits[m];
-            hi_tab[v] = o;
-        }
-    }
-    for (int i = tid; i < ADJ_GROUP_WARPS * ADJ_GROUP_MAX_BITS * 4; i += ADJ_GROUP_THREADS) sacc[i] = 0.0;
-    __syncthreads();
-    const int lomask = (1 << nlo) - 1;
-    for (uint64_t g = blockIdx.x; g < p.ngroups; g += gridDim.x) {
-        uint64_t base = g;
-        for (int m = 0; m < p.nbits; ++m) base = insert_zero(base, p.bits[m]);
-        for (int i = tid; i < T; i += ADJ_GROUP_THREADS) {
-            const uint64_t o = base | lo_tab[i & lomask] | hi_tab[i >> nlo];
-            sf[i] = phi[o];
-            sl[i] = lam[o];
-        }
-        __syncthreads();
-        for (int w = 0; w < p.nwires; ++w) {
-            const AdjGroupWireF& W = p.w[w];
-            const int lb = W.lb;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int q = tid; q < (T >> 1); q += ADJ_GROUP_THREADS) {
-                const int i0 = ((q >> lb) << (lb + 1)) | (q & ((1 << lb) - 1));
-                const int i1 = i0 | (1 << lb);
-                const float2 f0 = sf[i0], f1 = sf[i1], l0 = sl[i0], l1 = sl[i1];
-                // Im(conj(a) b) = a.x b.y - a.y b.x, Re(conj(a) b) = a.x b.x + a.y b.y
-                const float i01 = fmaf(l0.x, f1.y, -l0.y * f1.x), i10 = fmaf(l1.x, f0.y, -l1.y * f0.x);
-                const float r01 = fmaf(l0.x, f1.x, l0.y * f1.y), r10 = fmaf(l1.x, f0.x, l1.y * f0.y);
-                const float i00 = fmaf(l0.x, f0.y, -l0.y * f0.x), i11 = fmaf(l1.x, f1.y, -l1.y * f1.x);
-                acc[0] += i01 + i10;     // X
-                acc[1] += r10 - r01;     // Y
-                acc[2] += i00 - i11;     // Z
-                acc[3] -= i00 + i11;     // global phase
-                sf[i0] = cmul_add(W.u[0], W.u[1], f0, W.u[2], W.u[3], f1);
-                sf[i1] = cmul_add(W.u[4], W.u[5], f0, W.u[6], W.u[7], f1);
-                sl[i0] = cmul_add(W.u[0], W.u[1], l0, W.u[2], W.u[3], l1);
-                sl[i1] = cmul_add(W.u[4], W.u[5], l0, W.u[6], W.u[7], l1);
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                if (W.row[m] < 0) continue;
-                float v = acc[m];
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-                if (lane == 0) sacc[(warp * ADJ_GROUP_MAX_BITS + w) * 4 + m] += (double)v;
-            }
-            __syncthreads();
-        }
-        for (int i = tid; i < T; i += ADJ_GROUP_THREADS) {
-            const uint64_t o = base | lo_tab[i & lomask] | hi_tab[i >> nlo];
-            phi[o] = sf[i];
-            lam[o] = sl[i];
-        }
-        __syncthreads();
-    }
-    for (int k = tid; k < p.nwires * 4; k += ADJ_GROUP_THREADS) {
-        const int w = k >> 2, m = k & 3;
-        if (p.w[w].row[m] < 0) continue;
-        double t = 0.0;
-        for (int v = 0; v < ADJ_GROUP_WARPS; ++v) t += sacc[(v * ADJ_GROUP_MAX_BITS + w) * 4 + m];
-        double* row = partial + (size_t)p.w[w].row[m] * p.nb;
-        row[blockIdx.x] = t;
-        for (int c = blockIdx.x + gridDim.x; c < p.nb; c += gridDim.x) row[c] = 0.0;
-    }
-}
-
-static int launch_adj_group_f32(qgpu_handle* h, float2* phi, float2* lam, const AdjGroupParamsF& p,
-                                double* partial) {
-    const size_t smem = adj_group_f32_smem(p.nbits);
-    QGPU_CUDA(smem_opt_in((const void*)k_adj_group_f32, adj_group_f32_smem(ADJ_GROUP_MAX_BITS)));
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adj_group_f32, ADJ_GROUP_THREADS, smem) != cudaSuccess || occ < 1)
-        occ = 1;
-    const uint64_t grid = std::max<uint64_t>(
-        1, std::min<uint64_t>({p.ngroups, (uint64_t)h->sm_count * occ, (uint64_t)p.nb}));
-    return adj_profiled(h, "k_adj_group_f32", 32.0 * (double)h->dim, [&]() -> int {
-        k_adj_group_f32<<<(unsigned)grid, ADJ_GROUP_THREADS, smem, h->stream>>>(phi, lam, p, partial);
-        QGPU_CHECK_LAUNCH("k_adj_group_f32");
-        h->launches++;
-        h->h2d_bytes += sizeof(p);
-        return QGPU_OK;
-    });
 }
 
 template <int K>
@@ -763,9 +447,73 @@ static int ham_from(const qgpu_handle* h, const double* a, const double* b, Ham*
     return QGPU_OK;
 }
 
+// A run of single-wire gates (op indices in reverse order) wire by wire: the bit of each wire, in
+// first-seen order, and its ops in reverse order.
+static void by_wire(const qgpu_op* ops, const std::vector<size_t>& run, int n,
+                    std::vector<int>* wires, std::vector<std::vector<size_t>>* gates) {
+    for (size_t gi : run) {
+        const int bit = n - 1 - ops[gi].target;
+        const size_t w = std::find(wires->begin(), wires->end(), bit) - wires->begin();
+        if (w == wires->size()) {
+            wires->push_back(bit);
+            gates->emplace_back();
+        }
+        (*gates)[w].push_back(gi);
+    }
+}
+
+// Undoes a run in grouped passes and records its gradient terms: op g's gradient is the sum over
+// terms[g] of coefficient x row sum.
+static int group_run(qgpu_handle* h, void* phi, void* lam, const qgpu_op* ops,
+                     const std::vector<int>& wires, const std::vector<std::vector<size_t>>& gates,
+                     double* partial, int nb, int* nrows,
+                     std::vector<std::vector<std::pair<int, double>>>* terms) {
+    std::vector<PauliRun> prs(wires.size());
+    std::vector<PauliFrame> frames(wires.size());
+    for (size_t w = 0; w < wires.size(); ++w) {
+        int st = pauli_run(ops, gates[w], h->n_qubits, &prs[w]);
+        if (st != QGPU_OK) return st;
+        frames[w] = pauli_frame(&prs[w]);
+    }
+    // runs of 2^low amplitudes load together: the longest ones that cost no further pass
+    const int tile = adj_group_tile_bits(h->precision);
+    auto passes = adj_group_passes(wires, h->n_qubits, tile, 2);
+    for (int low = 5; low > 2; --low) {
+        auto wider = adj_group_passes(wires, h->n_qubits, tile, low);
+        if (wider.size() == passes.size()) {
+            passes.swap(wider);
+            break;
+        }
+    }
+    for (const auto& pass : passes) {
+        std::vector<AdjGroupWire> ws;
+        int row_i = -1;
+        for (size_t w : pass.second) {
+            AdjGroupWire gw;
+            gw.bit = wires[w];
+            gw.frame = frames[w];
+            int kind_row[5];
+            for (int m = 1; m <= 3; ++m) gw.row[m - 1] = kind_row[m] = prs[w].need[m] ? (*nrows)++ : -1;
+            if (prs[w].need[4] && row_i < 0) row_i = (*nrows)++;
+            kind_row[4] = row_i;
+            for (const auto& r : prs[w].rots)
+                for (int m = 1; m <= 4; ++m)
+                    if (r.second[m] != 0.0) (*terms)[r.first].emplace_back(kind_row[m], r.second[m]);
+            ws.push_back(gw);
+        }
+        const int st = adj_profiled(
+            h, h->precision == QGPU_C64 ? "k_adj_group_f32" : "k_adj_group",
+            4.0 * h->amp_bytes * (double)h->dim, [&]() {
+            return adj_group_pass(h, phi, lam, pass.first, ws, row_i, partial, nb);
+        });
+        if (st != QGPU_OK) return st;
+    }
+    return QGPU_OK;
+}
+
 // The adjoint sweep of a complex64 handle (the forward pass has run on the register): phi and
 // lambda as complex64 work vectors, every run of single-wire gates in grouped passes
-// (k_adj_group_f32), runs of multi-wire gates undone as one index gather (k_linperm) or through
+// (adj_group.cu), runs of multi-wire gates undone as one index gather (k_linperm) or through
 // the register-tile passes. The gradients are formed on the host from the Pauli sums, as in the
 // complex128 sweep.
 static int adjoint_sweep_c64(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const Ham& H,
@@ -828,52 +576,11 @@ static int adjoint_sweep_c64(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, c
     std::vector<size_t> run;  // op indices of the current single-wire run, in reverse order
     auto flush_run = [&]() -> int {
         if (run.empty()) return QGPU_OK;
-        std::vector<int> wires;                  // bit of each wire, in first-seen order
-        std::vector<std::vector<size_t>> gates;  // per wire, its ops in reverse order
-        for (size_t gi : run) {
-            const int bit = h->n_qubits - 1 - ops[gi].target;
-            size_t w = std::find(wires.begin(), wires.end(), bit) - wires.begin();
-            if (w == wires.size()) {
-                wires.push_back(bit);
-                gates.emplace_back();
-            }
-            gates[w].push_back(gi);
-        }
+        std::vector<int> wires;
+        std::vector<std::vector<size_t>> gates;
+        by_wire(ops, run, h->n_qubits, &wires, &gates);
         run.clear();
-        std::vector<PauliRun> prs(wires.size());
-        for (size_t w = 0; w < wires.size(); ++w) {
-            int s3 = pauli_run(ops, gates[w], h->n_qubits, &prs[w]);
-            if (s3 != QGPU_OK) return s3;
-        }
-        for (const auto& pass : adj_group_passes(wires, h->n_qubits, ADJ_GROUP_MAX_BITS)) {
-            AdjGroupParamsF p;
-            std::memset(&p, 0, sizeof(p));
-            for (int b = 0; b < 64; ++b)
-                if ((pass.first >> b) & 1ull) p.bits[p.nbits++] = b;
-            p.ngroups = h->dim >> p.nbits;
-            p.nb = nb;
-            p.nwires = (int)pass.second.size();
-            for (int c = 0; c < p.nwires; ++c) {
-                const size_t w = pass.second[c];
-                AdjGroupWireF& gw = p.w[c];
-                gw.lb = (int)(std::find(p.bits, p.bits + p.nbits, wires[w]) - p.bits);
-                int kind_row[5] = {-1, -1, -1, -1, -1};
-                for (int m = 1; m <= 4; ++m) {
-                    gw.row[m - 1] = -1;
-                    if (prs[w].need[m]) gw.row[m - 1] = kind_row[m] = nrows++;
-                }
-                for (int e = 0; e < 4; ++e) {
-                    gw.u[2 * e] = (float)prs[w].undo[e].real();
-                    gw.u[2 * e + 1] = (float)prs[w].undo[e].imag();
-                }
-                for (const auto& r : prs[w].rots)
-                    for (int m = 1; m <= 4; ++m)
-                        if (r.second[m] != 0.0) terms[r.first].emplace_back(kind_row[m], r.second[m]);
-            }
-            int s2 = launch_adj_group_f32(h, phi, lam, p, partial);
-            if (s2 != QGPU_OK) return s2;
-        }
-        return QGPU_OK;
+        return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &terms);
     };
     for (size_t gi = n_ops; gi-- > 0;) {
         const qgpu_op& op = ops[gi];
@@ -1048,17 +755,9 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
     std::vector<size_t> run;  // op indices of the current single-wire run, in reverse order
     auto flush_run = [&]() -> int {
         if (run.empty()) return QGPU_OK;
-        std::vector<int> wires;                  // bit of each wire, in first-seen order
-        std::vector<std::vector<size_t>> gates;  // per wire, its ops in reverse order
-        for (size_t gi : run) {
-            const int bit = h->n_qubits - 1 - ops[gi].target;
-            size_t w = std::find(wires.begin(), wires.end(), bit) - wires.begin();
-            if (w == wires.size()) {
-                wires.push_back(bit);
-                gates.emplace_back();
-            }
-            gates[w].push_back(gi);
-        }
+        std::vector<int> wires;
+        std::vector<std::vector<size_t>> gates;
+        by_wire(ops, run, h->n_qubits, &wires, &gates);
         run.clear();
         // Pauli-sum passes take less arithmetic (one 2x2 update per vector per wire instead of
         // one per gate) and win once the vectors live in HBM; with the vectors in L2 (up to 21
@@ -1066,55 +765,14 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
         // 24 qubits: 35.1 against 29.9 ms). Tuning knob QGPU_ADJ_PAULI: 0 / 1 forces either.
         const char* pk = std::getenv("QGPU_ADJ_PAULI");  // read per call (tests force either)
         const int pauli_knob = (pk && pk[0] == '0') ? 0 : (pk && pk[0] == '1') ? 1 : -1;
-        // Grouped passes (k_adj_group: the wires of a run in tiles of up to 11 bits, one pass
-        // per tile) up to 22 qubits; QGPU_ADJ_GROUP=0 / 1 (read per call) forces them off / on.
-        // Measured on GB300 (4-layer ansatz, energy + gradient): 20 qubits 5.23 against 6.34 ms
-        // (30 launches instead of 200), 22 qubits 7.72 against 7.76 ms, 24 qubits 31.8 against
-        // 29.8 ms: a wire's float-pair sums and undo keep the FMA pipe 64 % busy for about as
-        // long as one streaming pass over both vectors takes, so from 23 qubits the per-wire
-        // passes (HBM-bound, the arithmetic hidden under the traffic) are kept.
-        // The batch autotuner's pick (h->adj_group) comes first.
+        // Grouped passes (adj_group.cu: the wires of a run in tiles of up to 10 bits, one pass per
+        // tile); QGPU_ADJ_GROUP=0 (read per call) selects one pass per wire. Measured on GB300
+        // (4-layer ansatz, energy + gradient, grouped against per-wire): 13 qubits 0.51 / 0.77 ms,
+        // 20 qubits 1.46 / 2.54 ms, 24 qubits 16.9 / 26.2 ms, 25 qubits 33.8 / 52.6 ms.
         const char* gk = std::getenv("QGPU_ADJ_GROUP");
-        const int forced = h->adj_group >= 0 ? h->adj_group : gk ? (gk[0] != '0' ? 1 : 0) : -1;
-        const bool group = pauli_knob != 0 && (forced >= 0 ? forced == 1 : h->n_qubits <= 22);
+        const bool group = pauli_knob != 0 && !(gk && gk[0] == '0');
         const bool pauli = pauli_knob >= 0 ? pauli_knob == 1 : h->n_qubits >= 22;
-        if (group) {
-            std::vector<PauliRun> prs(wires.size());
-            for (size_t w = 0; w < wires.size(); ++w) {
-                int s3 = pauli_run(ops, gates[w], h->n_qubits, &prs[w]);
-                if (s3 != QGPU_OK) return s3;
-            }
-            for (const auto& pass : adj_group_passes(wires, h->n_qubits, ADJ_GROUP_MAX_BITS)) {
-                const uint64_t mask = pass.first;
-                const std::vector<size_t>& chosen = pass.second;
-                AdjGroupParams p;
-                std::memset(&p, 0, sizeof(p));
-                for (int b = 0; b < 64; ++b)
-                    if ((mask >> b) & 1ull) p.bits[p.nbits++] = b;
-                p.ngroups = h->dim >> p.nbits;
-                p.nb = nb;
-                p.nwires = (int)chosen.size();
-                for (int c = 0; c < p.nwires; ++c) {
-                    const size_t w = chosen[c];
-                    AdjGroupWire& gw = p.w[c];
-                    gw.lb = (int)(std::find(p.bits, p.bits + p.nbits, wires[w]) - p.bits);
-                    int kind_row[5] = {-1, -1, -1, -1, -1};
-                    for (int m = 1; m <= 4; ++m) {
-                        gw.row[m - 1] = -1;
-                        if (prs[w].need[m]) gw.row[m - 1] = kind_row[m] = nrows++;
-                    }
-                    const std::array<cd, 4>& undo = prs[w].undo;
-                    const DevStep ds = dense_step(undo[0], undo[1], undo[2], undo[3]);
-                    std::memcpy(gw.pk, ds.pk, sizeof(gw.pk));
-                    for (const auto& r : prs[w].rots)
-                        for (int m = 1; m <= 4; ++m)
-                            if (r.second[m] != 0.0) terms[r.first].emplace_back(kind_row[m], r.second[m]);
-                }
-                int s2 = launch_adj_group(h, phi, lam, p, partial);
-                if (s2 != QGPU_OK) return s2;
-            }
-            return QGPU_OK;
-        }
+        if (group) return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &terms);
         if (tile_bits == 1 && pauli) {
             // One pass per wire: the sums <lambda| s |phi> for the Paulis s the run's rotations
             // need, all taken before any of its gates is undone, then the whole run undone as one

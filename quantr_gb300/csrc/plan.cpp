@@ -1382,13 +1382,50 @@ qgpu_op inverse_op(const qgpu_op& op) {
     return r;
 }
 
+PauliFrame pauli_frame(PauliRun* run) {
+    const std::array<cd, 4>& m = run->undo;  // m00 m01 m10 m11
+    PauliFrame f;
+    f.c = std::abs(m[0]);
+    f.s = std::abs(m[1]);
+    const double r = std::hypot(f.c, f.s);
+    f.c /= r;
+    f.s /= r;
+    auto unit = [](cd z) { return z / std::abs(z); };
+    if (m[1] == cd(0.0, 0.0)) {  // diagonal
+        f.c = 1.0;
+        f.s = 0.0;
+        f.rho1 = unit(m[3] / m[0]);
+    } else if (m[0] == cd(0.0, 0.0)) {  // e^{i a} [[0, -rho1], [1, 0]]
+        f.c = 0.0;
+        f.s = 1.0;
+        f.rho1 = unit(-m[1] / m[2]);
+    } else {
+        f.rho1 = unit(-m[1] / unit(m[0]));
+        f.rho2 = unit(m[2] / unit(m[0]));
+    }
+    for (int k = 0; k < 5; ++k) run->need[k] = false;
+    for (auto& rot : run->rots) {
+        std::array<double, 5>& q = rot.second;
+        const double x = q[1] * f.rho1.real() - q[2] * f.rho1.imag();
+        const double y = q[1] * f.rho1.imag() + q[2] * f.rho1.real();
+        q[1] = x;
+        q[2] = y;
+        for (int k = 1; k <= 4; ++k) {
+            if (std::fabs(q[k]) <= 4.5e-16) q[k] = 0.0;
+            run->need[k] = run->need[k] || q[k] != 0.0;
+        }
+    }
+    return f;
+}
+
 std::vector<std::pair<uint64_t, std::vector<size_t>>> adj_group_passes(const std::vector<int>& bits,
-                                                                       int n, int max_bits) {
+                                                                       int n, int max_bits,
+                                                                       int low_bits) {
     std::vector<size_t> order(bits.size());
     for (size_t w = 0; w < order.size(); ++w) order[w] = w;
     std::sort(order.begin(), order.end(), [&](size_t x, size_t y) { return bits[x] < bits[y]; });
     const int kmax = std::min(n, max_bits);
-    const uint64_t low = (1ull << std::min(n, 5)) - 1;
+    const uint64_t low = (1ull << std::min(n, low_bits)) - 1;
     std::vector<std::pair<uint64_t, std::vector<size_t>>> out;
     size_t i = 0;
     while (i < order.size()) {

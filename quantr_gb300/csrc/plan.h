@@ -53,14 +53,26 @@ struct PauliRun {
 // gw: the run's op indices into ops, in reverse order (gw[0] the run's last gate).
 int pauli_run(const qgpu_op* ops, const std::vector<size_t>& gw, int n, PauliRun* out);
 
+// The undo of a run, undo = e^{i a} diag(1, rho2) [[c, -s], [s, c]] diag(1, rho1): the phase e^{i a}
+// (common to both vectors of a sweep) is dropped. Conjugating by diag(1, rho1) mixes X and Y only,
+// so a rotation's coefficients are turned into those of the sums taken after it: for a run that
+// ends in Ry, Rz or Rz alone no X sum is left. Coefficients up to 4.5e-16 in magnitude (the
+// rounding of the products they come from) are dropped.
+struct PauliFrame {
+    double c = 1.0, s = 0.0;
+    cd rho1 = 1.0, rho2 = 1.0;
+};
+PauliFrame pauli_frame(PauliRun* run);
+
 // The passes of a grouped adjoint sweep (the runs of single-wire gates of many wires per pass):
 // wire bits in ascending order, each pass a tile of at most `max_bits` index bits that always
-// holds bits 0..4 (32 consecutive amplitudes per load) and is filled up with the lowest other
-// bits. Returns per pass the tile mask and the wires (indices into `bits`) it takes; every wire
+// holds the `low_bits` lowest bits (runs of consecutive amplitudes per load) and is filled up with
+// the lowest other bits. Returns per pass the tile mask and the wires (indices into `bits`) it takes; every wire
 // lands in exactly one pass.
 constexpr int ADJ_GROUP_TILE_BITS = 11;
 std::vector<std::pair<uint64_t, std::vector<size_t>>> adj_group_passes(const std::vector<int>& bits,
-                                                                       int n, int max_bits);
+                                                                       int n, int max_bits,
+                                                                       int low_bits = 5);
 // Whether ops (CNot, X, Swap only), applied in order, form an affine index map y -> A y + b over
 // GF(2); if so, the gather tables of its inverse h for one out-of-place pass dst[y] = src[h(y)]:
 // h(y) = *d xor tabs[c * 256 + byte c of y] over the 8-bit chunks c of y.

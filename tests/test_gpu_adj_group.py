@@ -1,0 +1,61 @@
+"""Grouped passes of the adjoint sweep (quantr_gb300/csrc/adj_group.cu) against the one-gate f64
+sweep (QGPU_MODE_F64), at the edges of their tiles, for runs whose undo needs every part of the
+frame: Y sums alone, X sums, both diagonals, a diagonal or antidiagonal undo, the -I sum.
+
+Tolerances: complex128 1e-11 (float pairs, the adjoint tests' bar between sweep forms is 1e-9);
+complex64 1e-4, the adjoint tests' bar.
+"""
+import numpy as np
+import pytest
+
+from quantr_gb300 import _native as nat
+from quantr_gb300 import gradients as GR
+from quantr_gb300.program import ProgramBuilder
+
+pytestmark = pytest.mark.gpu
+
+RUNS = {
+    "ry_rz": ["Ry", "Rz"],
+    "rz_ry": ["Rz", "Ry"],
+    "rx": ["Rx"],
+    "zyz": ["Rz", "Ry", "Rz"],
+    "diagonal": ["Rz", "S", "T"],
+    "antidiagonal": ["X", "Rz", "Y"],
+    "phase": ["Phase", "Rx", "H"],
+    "mixed": ["H", "Ry", "T", "Rx", "Phase", "X90"],
+}
+
+
+@pytest.fixture(autouse=True)
+def _lib(gpu_lib):
+    yield
+
+
+def _program(n, run, seed):
+    r = np.random.default_rng(seed)
+    b = ProgramBuilder(n)
+    for _ in range(2):
+        for w in range(n):
+            if run == "some" and w % 3 == 1:
+                continue
+            for g in RUNS[list(RUNS)[w % len(RUNS)] if run == "some" else run]:
+                b.add(g, w, (), param=r.uniform(-3, 3) if g in ("Rx", "Ry", "Rz", "Phase") else 0.0)
+        for w in range(n - 1):
+            b.add("CNot", w + 1, (w,))
+    return b.build(), r.standard_normal(n), r.standard_normal(n)
+
+
+# 1, 2: below a round's bits; 8/9: thread bits / register bits; 11/12: one tile / two passes;
+# 14: a last round of one wire
+@pytest.mark.parametrize("n,run", [(1, "mixed"), (2, "zyz"), (3, "rx"), (5, "phase"), (8, "ry_rz"),
+                                   (9, "mixed"), (11, "zyz"), (12, "rz_ry"), (13, "diagonal"),
+                                   (13, "antidiagonal"), (14, "some"), (17, "mixed"), (21, "ry_rz")])
+@pytest.mark.parametrize("precision", [nat.QGPU_C128, nat.QGPU_C64])
+def test_grouped_passes_against_the_f64_sweep(monkeypatch, n, run, precision):
+    monkeypatch.setenv("QGPU_ADJ_GROUP", "1")
+    prog, a, b = _program(n, run, n)
+    e, g = GR.energy_and_gradient(nat.Handle(n, precision), prog, a, b)
+    re, rg = GR.energy_and_gradient(nat.Handle(n, nat.QGPU_C128, nat.QGPU_MODE_F64), prog, a, b)
+    tol = 1e-11 if precision == nat.QGPU_C128 else 1e-4
+    assert abs(e - re) <= tol
+    assert np.max(np.abs(g - rg)) <= tol
