@@ -1402,7 +1402,14 @@ PauliFrame pauli_frame(PauliRun* run) {
     } else {
         f.rho1 = unit(-m[1] / unit(m[0]));
         f.rho2 = unit(m[2] / unit(m[0]));
+        if (f.rho2.real() < 0.0) {  // the sign of s that leaves rho2 near 1 (Ry next to Rz: 1)
+            f.s = -f.s;
+            f.rho1 = -f.rho1;
+            f.rho2 = -f.rho2;
+        }
     }
+    if (std::abs(f.rho1 - 1.0) <= 4.5e-16) f.rho1 = 1.0;
+    if (std::abs(f.rho2 - 1.0) <= 4.5e-16) f.rho2 = 1.0;
     for (int k = 0; k < 5; ++k) run->need[k] = false;
     for (auto& rot : run->rots) {
         std::array<double, 5>& q = rot.second;
