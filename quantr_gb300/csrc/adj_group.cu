@@ -40,7 +40,7 @@ struct AgWire {
     int lb;              // tile bit
     int row[3];          // partial rows of its X, Y, Z sums (-1: not needed)
     float4 rho1, rho2;   // (re_h, re_l, im_h, im_l) of its D1 and D2
-    u64 c[16];           // R as Dot2 terms: out0 = c0 a + c1 b, out1 = c2 a + c3 b (hi, lo, -hi, -lo)
+    u64 c[16];           // R as Dot2 terms: out0 = c0 a + c1 b, out1 = c2 a + c3 b (hi, -third, -hi, -lo)
 };
 struct AgParams {
     uint64_t ngroups;
@@ -57,6 +57,7 @@ struct AgParams {
     int d1, d2, xsum, zsum;
     int nb;              // row length of partial (>= the grid)
     int ins[AG_SLOTS];   // per round, its bits in ascending order
+    float4 dt1[256];     // D1's factor for the tile bits in the thread index
     AgWire w[AG_SLOTS];  // round r: wires r * R ..., filled up with other tile bits
 };
 
@@ -90,23 +91,32 @@ __device__ __forceinline__ void ag_acc3(AgF3& v, float h, float l) {
 }
 __device__ __forceinline__ u64 pneg(u64 a) { return a ^ 0x8000000080000000ull; }
 
+// Product of complex constants in float pairs, (re_h, re_l, im_h, im_l).
+__device__ __forceinline__ float4 ag_cmul(float4 a, float4 v) {
+    const u64 c[8] = {p2(v.x, v.x), p2(v.y, v.y), p2(-v.x, -v.x), p2(-v.y, -v.y),
+                      p2(-v.z, v.z), p2(-v.w, v.w), p2(v.z, -v.z), p2(v.w, -v.w)};
+    const u64 h = p2(a.x, a.z), l = p2(a.y, a.w);
+    PDot2 d;
+    d.first(c, h, l);
+    d.add(c + 4, pswap(h), pswap(l));
+    u64 rh, rl;
+    d.result(rh, rl);
+    float4 r;
+    up2(rh, r.x, r.z);
+    up2(rl, r.y, r.w);
+    return r;
+}
+
 struct AgFF {
     using S = double2;
     using V = ffp;
     using C = float4;  // complex constant (re_h, re_l, im_h, im_l)
+    static __device__ __forceinline__ C combine(C a, C b) { return ag_cmul(a, b); }
     static constexpr int R = 2, TBITS = 7, CTAS = 4;  // TBITS: tile bits in the thread index
     static __device__ __forceinline__ V get(S a) { return ffr_load(a); }
     static __device__ __forceinline__ S put(const V& v) { return ffr_store(v); }
     static __device__ __forceinline__ V swap(const V& v) { return V{pswap(v.h), pswap(v.l)}; }
     static __device__ __forceinline__ V neg(const V& v) { return V{pneg(v.h), pneg(v.l)}; }
-    static __device__ __forceinline__ C constant(float4 c) { return c; }
-    static __device__ __forceinline__ V value(C c) { return V{p2(c.x, c.z), p2(c.y, c.w)}; }
-    static __device__ __forceinline__ C constant_of(const V& v) {
-        C c;
-        up2(v.h, c.x, c.z);
-        up2(v.l, c.y, c.w);
-        return c;
-    }
     static __device__ __forceinline__ void mul(V& a, C v) {
         const u64 c[8] = {p2(v.x, v.x), p2(v.y, v.y), p2(-v.x, -v.x), p2(-v.y, -v.y),
                           p2(-v.z, v.z), p2(-v.w, v.w), p2(v.z, -v.z), p2(v.w, -v.w)};
@@ -118,11 +128,11 @@ struct AgFF {
     static __device__ __forceinline__ void real(V& a, V& b, const u64* c) {
         PDot2 d;
         V o0, o1;
-        d.first(c + 0, a.h, a.l);
-        d.add(c + 4, b.h, b.l);
+        d.first3(c + 0, a.h, a.l);
+        d.add3(c + 4, b.h, b.l);
         d.result(o0.h, o0.l);
-        d.first(c + 8, a.h, a.l);
-        d.add(c + 12, b.h, b.l);
+        d.first3(c + 8, a.h, a.l);
+        d.add3(c + 12, b.h, b.l);
         d.result(o1.h, o1.l);
         a = o0;
         b = o1;
@@ -187,7 +197,7 @@ struct AgZFF {
 struct AgF32 {
     using S = float2;
     using V = u64;
-    using C = float2;
+    using C = float4;
     static constexpr int R = 3, TBITS = 8, CTAS = 3;
     static __device__ __forceinline__ V get(S a) { return p2(a.x, a.y); }
     static __device__ __forceinline__ S put(V v) {
@@ -197,14 +207,30 @@ struct AgF32 {
     }
     static __device__ __forceinline__ V swap(V v) { return pswap(v); }
     static __device__ __forceinline__ V neg(V v) { return pneg(v); }
-    static __device__ __forceinline__ C constant(float4 c) { return make_float2(c.x, c.z); }
-    static __device__ __forceinline__ V value(C c) { return get(c); }
-    static __device__ __forceinline__ C constant_of(V v) { return put(v); }
+    // a b rounded to f32 (a factor per tile index: its rounding differs from one to the next)
+    static __device__ __forceinline__ C combine(C a, C b) {
+        const u64 bs = p2(-b.z, b.x), bl = p2(-b.w, b.y), bh = p2(b.x, b.z), bm = p2(b.y, b.w);
+        u64 r = pmul(p2(a.y, a.y), bh);
+        r = pfma(p2(a.w, a.w), bs, r);
+        r = pfma(p2(a.x, a.x), bm, r);
+        r = pfma(p2(a.z, a.z), bl, r);
+        r = pfma(p2(a.x, a.x), bh, r);
+        r = pfma(p2(a.z, a.z), bs, r);
+        C c = make_float4(0.f, 0.f, 0.f, 0.f);
+        up2(r, c.x, c.z);
+        return c;
+    }
     static __device__ __forceinline__ void mul(V& a, C c) {
-        a = pfma(p2(c.x, c.x), a, pmul(p2(-c.y, c.y), pswap(a)));
+        const u64 r = pmul(p2(c.x, c.x), a), i = pmul(p2(c.z, c.z), a);
+        float rx, ry, ix, iy;
+        up2(r, rx, ry);
+        up2(i, ix, iy);
+        a = p2(rx - iy, ry + ix);
     }
     static __device__ __forceinline__ void real(V& a, V& b, const u64* c) {
-        const V o0 = pfma(c[0], a, pmul(c[4], b)), o1 = pfma(c[8], a, pmul(c[12], b));
+        // c + 3: minus the low parts, which keep all but the amplitudes from being rounded to f32
+        const V o0 = pfma(c[0], a, pfma(c[4], b, pneg(pfma(c[3], a, pmul(c[7], b)))));
+        const V o1 = pfma(c[8], a, pfma(c[12], b, pneg(pfma(c[11], a, pmul(c[15], b)))));
         a = o0;
         b = o1;
     }
@@ -311,7 +337,10 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
     const int T = 1 << p.nbits;
     // offsets and diagonal factors of this thread's tile bits and of the register bits
     uint64_t off_t = 0;
-    V d1v = P::value(P::constant(make_float4(1.f, 0.f, 0.f, 0.f))), d2v = d1v;
+    C dt1 = p.dt1[t];
+    // (kept in registers: a constant indexed by the thread is read lane by lane)
+    asm volatile("" : "+f"(dt1.x), "+f"(dt1.y), "+f"(dt1.z), "+f"(dt1.w));
+    C dt2 = make_float4(1.f, 0.f, 0.f, 0.f);
     for (int m = 0; m < p.nbits && m < AG_TBITS; ++m)
         if ((t >> m) & 1) off_t |= 1ull << p.bits[m];
     uint64_t off_j[AG_RBITS] = {0, 0, 0};
@@ -320,25 +349,23 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
         if (AG_TBITS + m < p.nbits) off_j[m] = 1ull << p.bits[AG_TBITS + m];
     for (int w = 0; w < p.nwires; ++w)
         if (p.w[w].lb < AG_TBITS && ((t >> p.w[w].lb) & 1)) {
-            P::mul(d1v, P::constant(p.w[w].rho1));
-            P::mul(d2v, P::constant(p.w[w].rho2));
+            dt2 = ag_cmul(dt2, p.w[w].rho2);
         }
-    const C dt1 = P::constant_of(d1v), dt2 = P::constant_of(d2v);
     if (t < AG_PER) {
-        V a = P::value(P::constant(make_float4(1.f, 0.f, 0.f, 0.f))), b = a;
+        C a = make_float4(1.f, 0.f, 0.f, 0.f), b = a;
         for (int w = 0; w < p.nwires; ++w)
             if (p.w[w].lb >= AG_TBITS && ((t >> (p.w[w].lb - AG_TBITS)) & 1)) {
-                P::mul(a, P::constant(p.w[w].rho1));
-                P::mul(b, P::constant(p.w[w].rho2));
+                a = ag_cmul(a, p.w[w].rho1);
+                b = ag_cmul(b, p.w[w].rho2);
             }
-        dj1[t] = P::constant_of(a);
-        dj2[t] = P::constant_of(b);
+        dj1[t] = a;
+        dj2[t] = b;
     }
     for (int i = t; i < (XS ? 2 : 1) * WIRES * AG_THREADS; i += AG_THREADS)
         red[i] = make_float2(0.f, 0.f);
     typename AgZ<P>::type z;
     z.clear();
-    if (t >= T && t < (1 << p.tile)) sf[ag_slot(t)] = sl[ag_slot(t)] = P::value(P::constant(make_float4(0.f, 0.f, 0.f, 0.f)));
+    if (t >= T && t < (1 << p.tile)) sf[ag_slot(t)] = sl[ag_slot(t)] = V{};
     __syncthreads();
     for (uint64_t g = blockIdx.x; g < p.ngroups; g += gridDim.x) {
         const uint64_t base = ag_base(p, g) | off_t;
@@ -352,9 +379,7 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
                 V f = P::get(phi[o]), l = P::get(lam[o]);
                 if (p.zsum) z.add(j, l, f);
                 if (p.d1) {
-                    V d = P::value(dt1);
-                    P::mul(d, dj1[j]);
-                    const C dc = P::constant_of(d);
+                    const C dc = P::combine(dt1, dj1[j]);
                     P::mul(f, dc);
                     P::mul(l, dc);
                 }
@@ -455,9 +480,7 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
                                    ((j & 4) ? off_j[2] : 0);
                 V f = sf[ag_slot(t + j * AG_THREADS)], l = sl[ag_slot(t + j * AG_THREADS)];
                 if (p.d2) {
-                    V d = P::value(dt2);
-                    P::mul(d, dj2[j]);
-                    const C dc = P::constant_of(d);
+                    const C dc = P::combine(dt2, dj2[j]);
                     P::mul(f, dc);
                     P::mul(l, dc);
                 }
@@ -522,13 +545,20 @@ static float4 ff_of(cd c) {
     return r;
 }
 static void real_term(u64* c, double v) {
-    const float h = (float)v, l = (float)(v - (double)h);
-    const float e[4] = {h, l, -h, -l};
+    const float h = (float)v, l = (float)(v - (double)h), third = (float)((v - (double)h) - (double)l);
+    const float e[4] = {h, -third, -h, -l};
     for (int k = 0; k < 4; ++k) {
         uint32_t b;
         std::memcpy(&b, &e[k], 4);
         c[k] = (u64)b | ((u64)b << 32);
     }
+}
+
+// x^2 + y^2 - 1 for a value near 0, exact but for its own rounding
+static double square_off(double x, double y) {
+    const double p = x * x, q = y * y, t = p + q, b = t - p;
+    const double e = (p - (t - b)) + (q - b);
+    return (t - 1.0) + (e + (std::fma(x, x, -p) + std::fma(y, y, -q)));
 }
 
 template <class P, bool XS>
@@ -555,7 +585,8 @@ int adj_group_tile_bits(int precision) {
 }
 
 int adj_group_pass(qgpu_handle* h, void* phi, void* lam, uint64_t mask,
-                   const std::vector<AdjGroupWire>& wires, int row_i, double* partial, int nb) {
+                   const std::vector<AdjGroupWire>& wires, int row_i, double* partial, int nb,
+                   double* drift) {
     AgParams p;
     std::memset(&p, 0, sizeof(p));
     for (int b = 0; b < 64; ++b)
@@ -585,11 +616,25 @@ int adj_group_pass(qgpu_handle* h, void* phi, void* lam, uint64_t mask,
         p.d2 = p.d2 || s.frame.rho2 != cd(1.0, 0.0);
         p.xsum = p.xsum || s.row[0] >= 0;
         p.zsum = p.zsum || s.row[2] >= 0;
-        real_term(w.c + 0, s.frame.c);
-        real_term(w.c + 4, -s.frame.s);
-        real_term(w.c + 8, s.frame.s);
-        real_term(w.c + 12, s.frame.c);
+        // c^2 + s^2 and the moduli of rho differ from 1 by f64 rounding, with a bias that 200 rotations
+        // turned into 1.5e-14 of both vectors' norms: the next rotation takes the drift out
+        const double c0 = s.frame.c - s.frame.c * *drift, s0 = s.frame.s - s.frame.s * *drift;
+        *drift += 0.5 * square_off(c0, s0) + 0.25 * square_off(s.frame.rho1.real(), s.frame.rho1.imag()) +
+                  0.25 * square_off(s.frame.rho2.real(), s.frame.rho2.imag());
+        real_term(w.c + 0, c0);
+        real_term(w.c + 4, -s0);
+        real_term(w.c + 8, s0);
+        real_term(w.c + 12, c0);
     }
+    const int tbits = h->precision == QGPU_C64 ? AgF32::TBITS : AgFF::TBITS;
+    // D1's factors in f64: as products of float pairs on the device their rounding added up over
+    // the layers of a circuit
+    std::vector<cd> dt((size_t)1 << tbits, cd(1.0, 0.0));
+    for (int c = 0; c < p.nwires && p.d1; ++c)
+        if (p.w[c].lb < tbits)
+            for (size_t t = 0; t < dt.size(); ++t)
+                if ((t >> p.w[c].lb) & 1) dt[t] *= wires[c].frame.rho1;
+    for (size_t t = 0; t < dt.size(); ++t) p.dt1[t] = ff_of(dt[t]);
     const int R = h->precision == QGPU_C64 ? AgF32::R : AgFF::R;
     p.tile = std::max(p.nbits, R);
     p.nrounds = (p.nwires + R - 1) / R;

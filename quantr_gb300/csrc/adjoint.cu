@@ -466,7 +466,7 @@ static void by_wire(const qgpu_op* ops, const std::vector<size_t>& run, int n,
 // terms[g] of coefficient x row sum.
 static int group_run(qgpu_handle* h, void* phi, void* lam, const qgpu_op* ops,
                      const std::vector<int>& wires, const std::vector<std::vector<size_t>>& gates,
-                     double* partial, int nb, int* nrows,
+                     double* partial, int nb, int* nrows, double* drift,
                      std::vector<std::vector<std::pair<int, double>>>* terms) {
     std::vector<PauliRun> prs(wires.size());
     std::vector<PauliFrame> frames(wires.size());
@@ -504,7 +504,7 @@ static int group_run(qgpu_handle* h, void* phi, void* lam, const qgpu_op* ops,
         const int st = adj_profiled(
             h, h->precision == QGPU_C64 ? "k_adj_group_f32" : "k_adj_group",
             4.0 * h->amp_bytes * (double)h->dim, [&]() {
-            return adj_group_pass(h, phi, lam, pass.first, ws, row_i, partial, nb);
+            return adj_group_pass(h, phi, lam, pass.first, ws, row_i, partial, nb, drift);
         });
         if (st != QGPU_OK) return st;
     }
@@ -540,6 +540,7 @@ static int adjoint_sweep_c64(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, c
     }
     std::vector<std::vector<std::pair<int, double>>> terms(n_ops);
     int nrows = 0;
+    double drift = 0.0;  // of both vectors' norms, by the rounding of the grouped passes' rotations
     std::vector<qgpu_op> seg;  // consecutive multi-wire gates, undone together
     float2* spare = nullptr;   // third vector for out-of-place index permutations
     auto flush_seg = [&]() -> int {
@@ -580,7 +581,7 @@ static int adjoint_sweep_c64(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, c
         std::vector<std::vector<size_t>> gates;
         by_wire(ops, run, h->n_qubits, &wires, &gates);
         run.clear();
-        return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &terms);
+        return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &drift, &terms);
     };
     for (size_t gi = n_ops; gi-- > 0;) {
         const qgpu_op& op = ops[gi];
@@ -709,6 +710,7 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
     // gradient of op g = sum over terms[g] of coefficient x (row sum)
     std::vector<std::vector<std::pair<int, double>>> terms(n_ops);
     int nrows = 0;
+    double drift = 0.0;  // of both vectors' norms, by the rounding of the grouped passes' rotations
     // reverse sweep
     std::vector<qgpu_op> seg;  // consecutive multi-wire gates, undone together
     double2* spare = nullptr;  // third vector for out-of-place index permutations
@@ -772,7 +774,7 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
         const char* gk = std::getenv("QGPU_ADJ_GROUP");
         const bool group = pauli_knob != 0 && !(gk && gk[0] == '0');
         const bool pauli = pauli_knob >= 0 ? pauli_knob == 1 : h->n_qubits >= 22;
-        if (group) return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &terms);
+        if (group) return group_run(h, phi, lam, ops, wires, gates, partial, nb, &nrows, &drift, &terms);
         if (tile_bits == 1 && pauli) {
             // One pass per wire: the sums <lambda| s |phi> for the Paulis s the run's rotations
             // need, all taken before any of its gates is undone, then the whole run undone as one

@@ -540,12 +540,13 @@ bool dg_build_image(const std::complex<double> M[16][16], uint32_t* bimg, int32_
 
 bool dg_supported(const qgpu_handle* h) {
     // tuning knobs, read per call: QGPU_DIGITS=0 keeps the float-pair kernels; digit runs are
-    // used from QGPU_DIGITS_MIN_QUBITS qubits (default 20: below that the register sits in L2
-    // and the two layout conversions cost more than the passes save)
+    // used from QGPU_DIGITS_MIN_QUBITS qubits (default 24: below that wide float-pair passes are
+    // faster, 20 brickwork layers at 20 / 22 / 23 / 24 qubits: 1.39 / 3.93 / 7.98 / 14.8 ms against
+    // 2.38 / 4.37 / 9.79 / 10.2 ms in digits)
     const char* e = std::getenv("QGPU_DIGITS");
     const char* m = std::getenv("QGPU_DIGITS_MIN_QUBITS");
     const int on = e ? std::atoi(e) : 1;
-    const int min_qubits = std::max(11, m ? std::atoi(m) : 20);
+    const int min_qubits = std::max(11, m ? std::atoi(m) : 24);
     return on != 0 && h->precision == QGPU_C128 && h->mode == QGPU_MODE_FAST &&
            (h->dim >> 4) % DG_M == 0 && h->n_qubits >= min_qubits;
 }

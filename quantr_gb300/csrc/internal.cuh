@@ -333,6 +333,25 @@ struct PDot2 {
         s = t;
         en = padd(psub(en, q), rn);
     }
+    // The same with constants of three floats, c[1] = -U_third (in place of U_lo, which no update
+    // reads): one operation more per term, and a gate's angle is exact to f64. Errors of the
+    // constants add up coherently over a circuit, those of the amplitudes do not.
+    __device__ __forceinline__ void first3(const u64* c, u64 xh, u64 xl) {
+        first(c, xh, xl);
+        en = pfma(c[1], xh, en);
+    }
+    __device__ __forceinline__ void add3(const u64* c, u64 xh, u64 xl) {
+        const u64 p = pmul(c[0], xh);
+        u64 rn = pfma(c[2], xh, p);
+        rn = pfma(c[2], xl, rn);
+        rn = pfma(c[3], xh, rn);
+        rn = pfma(c[1], xh, rn);
+        const u64 t = padd(s, p);  // TwoSum(s, p)
+        const u64 bb = psub(t, s);
+        const u64 q = padd(psub(s, psub(t, bb)), psub(p, bb));
+        s = t;
+        en = padd(psub(en, q), rn);
+    }
     __device__ __forceinline__ void result(u64& h, u64& l) const {  // FastTwoSum(s, -en)
         h = psub(s, en);
         l = psub(psub(s, h), en);

@@ -930,9 +930,306 @@ DevStep dense_step(cd u00, cd u01, cd u10, cd u11) {
     return s;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Wide passes: list scheduling. A pass takes, in program order, every step whose bits fit its tile
+// and that commutes with the steps passed over so far (they reach no bit that one of them
+// writes, and write none that one of them reads); its steps are then put into rounds of a few
+// bits in the same way. Steps read controls and phase bits anywhere in the index. X, CNot and Swap
+// need no round: they are carried out as soon as nothing holds them back.
+// ---------------------------------------------------------------------------------------------
+namespace {
+
+struct WideItem {
+    WideStep ws;
+    uint64_t need = 0;     // bits that must be in the tile, and in the step's round
+    uint64_t write = 0;    // bits it changes
+    uint64_t read = 0;     // other bits it depends on
+    int consts = 0;
+    enum Kind { PRE, ROT, PAIR, MOVE, OTHER } kind = OTHER;
+};
+
+// U = e^{i a} diag(1, rho2) [[c, -s], [s, c]] diag(1, rho1) to within `tol` in every entry.
+bool split_unitary(const cd u[4], PauliFrame* f, cd* phase) {
+    PauliRun r;
+    r.undo = {u[0], u[1], u[2], u[3]};
+    if (std::abs(u[0]) + std::abs(u[1]) == 0.0) return false;
+    if (u[1] == cd(0.0, 0.0) && (u[0] == cd(0.0, 0.0) || u[2] != cd(0.0, 0.0))) return false;
+    if (u[0] == cd(0.0, 0.0) && u[2] == cd(0.0, 0.0)) return false;
+    if (u[1] != cd(0.0, 0.0) && u[2] == cd(0.0, 0.0)) return false;
+    *f = pauli_frame(&r);
+    const cd lead = f->c != 0.0 ? u[0] : u[2];
+    *phase = lead / std::abs(lead);
+    const cd v[4] = {*phase * f->c, -*phase * f->s * f->rho1, *phase * f->rho2 * f->s,
+                     *phase * f->rho2 * f->c * f->rho1};
+    for (int k = 0; k < 4; ++k)
+        if (!(std::abs(v[k] - u[k]) <= 6.7e-16)) return false;
+    return true;
+}
+
+DevStep phase_step(int bit, cd rho) {
+    DevStep s = blank_step(ST_PHASE);
+    s.cm = 1ull << bit;
+    set_entry(s, 0, rho);
+    set_packed(s, &rho);
+    return s;
+}
+
+// Float pairs: an unconditional dense step costs 43 packed operations per amplitude, a real one 21
+// and a phase on one bit value 10.5. Unitary dense steps (and diagonal ones) become real steps
+// and phases; their common phases are collected and go with the last of them.
+void wide_items(const HStep& h, const PlanOptions& opt, std::vector<WideItem>* out, cd* phase,
+                int* phase_at) {
+    auto add = [&](const DevStep& s, int b0, int b1, int pair) {
+        WideItem it;
+        it.ws.s = s;
+        it.ws.bit[0] = b0;
+        it.ws.bit[1] = b1;
+        it.ws.pair = pair;
+        if (b0 >= 0) it.need |= 1ull << b0;
+        if (b1 >= 0) it.need |= 1ull << b1;
+        const bool diag = s.type == ST_PHASE || s.type == ST_DIAG || s.type == ST_TABLE;
+        it.write = diag ? 0 : it.need;
+        it.read = s.cm | (diag ? it.need : 0);
+        const bool ff = opt.policy == POL_FF;
+        switch (s.type) {
+            case ST_REAL: it.consts = ff ? 16 : 8; break;
+            case ST_DENSE: it.consts = ff ? 32 : 16; break;
+            case ST_PHASE: it.consts = s.unit ? 0 : ff ? 8 : 4; break;
+            case ST_DIAG: it.consts = s.unit ? 0 : ff ? 16 : 8; break;
+            case ST_DENSE4: it.consts = ff ? 128 : 32; break;
+            case ST_TABLE:
+                it.consts = s.nfields;
+                for (int f = 0; f < s.nfields; ++f)
+                    it.read |= ((1ull << s.tab_width[f]) - 1ull) << s.tab_shift[f];
+                break;
+            default: break;
+        }
+        const bool cx = s.type == ST_PERM && s.anti && s.u0 == 0 && s.u1 == 0 && popcount64(s.cm) <= 1;
+        if (s.type == ST_SWAP || cx) it.kind = WideItem::MOVE;
+        else if (s.type == ST_DENSE4) it.kind = WideItem::PAIR;
+        else if ((s.type == ST_REAL || s.type == ST_DENSE) && s.cm == 0) it.kind = WideItem::ROT;
+        else if (s.type == ST_PHASE && !s.unit && b0 >= 0 && s.cm == 1ull << b0) it.kind = WideItem::PRE;
+        out->push_back(it);
+    };
+    const DevStep& s = h.s;
+    if (opt.policy == POL_FF && s.cm == 0 && (s.type == ST_DENSE || (s.type == ST_DIAG && !h.unit))) {
+        cd u[4];
+        int bit = h.need[0];
+        if (s.type == ST_DENSE) {
+            for (int k = 0; k < 4; ++k) u[k] = cd(s.d[2 * k], s.d[2 * k + 1]);
+        } else {
+            bit = s.fb;
+            u[0] = cd(s.d[0], s.d[1]);
+            u[1] = u[2] = 0.0;
+            u[3] = cd(s.d[2], s.d[3]);
+        }
+        PauliFrame f;
+        cd ph;
+        if (split_unitary(u, &f, &ph)) {
+            *phase *= ph;
+            if (f.rho1 != cd(1.0, 0.0)) add(phase_step(bit, f.rho1), bit, -1, -1);
+            if (f.s != 0.0) {
+                DevStep r = blank_step(ST_REAL);
+                const cd e[4] = {f.c, -f.s, f.s, f.c};
+                for (int k = 0; k < 4; ++k) set_entry(r, k, e[k]);
+                set_packed(r, e);
+                add(r, bit, -1, -1);
+            }
+            if (f.rho2 != cd(1.0, 0.0)) add(phase_step(bit, f.rho2), bit, -1, -1);
+            *phase_at = bit;
+            return;
+        }
+    }
+    if (s.type == ST_DIAG) add(s, s.fb, -1, -1);
+    else if (s.type == ST_PHASE && !s.unit && popcount64(s.cm) == 1)
+        add(s, __builtin_ctzll(s.cm), -1, -1);  // (T: one bit, its register's)
+    else if (s.type == ST_DENSE4) add(s, h.need[0], h.need[1], (int)s.tab_off[0]);
+    else add(s, h.need[0], h.need[1], -1);
+}
+
+// Passes for steps [begin, end); false when they are not fewer than `limit`.
+bool wide_schedule(const std::vector<HStep>& steps, size_t begin, size_t end, int n,
+                   const PlanOptions& opt, size_t limit, std::vector<WidePass>* out) {
+    std::vector<WideItem> items;
+    items.reserve(end - begin);
+    cd phase(1.0, 0.0);
+    int phase_at = -1;
+    for (size_t i = begin; i < end; ++i) wide_items(steps[i], opt, &items, &phase, &phase_at);
+    if (phase_at >= 0 && phase != cd(1.0, 0.0)) {
+        const cd ph = phase / std::abs(phase);  // both values of one bit
+        DevStep s = blank_step(ST_DIAG);
+        s.fb = (uint8_t)phase_at;
+        const cd e[2] = {ph, ph};
+        set_entry(s, 0, ph);
+        set_entry(s, 1, ph);
+        set_packed(s, e);
+        HStep h;
+        h.s = s;
+        h.unit = true;  // (taken as it is)
+        wide_items(h, opt, &items, &phase, &phase_at);
+    }
+    const int width = std::min(n, opt.wide_bits);
+    const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1ull;
+    const uint64_t low = (1ull << std::min(n, opt.wide_low)) - 1ull;
+    std::vector<char> done(items.size(), 0);
+    size_t left = items.size(), first = 0;
+    while (left) {
+        if (out->size() + 1 >= limit) return false;
+        uint64_t tile = low, bw = 0, br = 0, outside = 0;
+        int consts = 0, nsteps = 0;
+        std::vector<size_t> taken;
+        while (first < items.size() && done[first]) ++first;
+        for (size_t i = first; i < items.size() && (bw & all) != all; ++i) {
+            if (done[i]) continue;
+            const WideItem& it = items[i];
+            bool ok = !(it.write & (bw | br)) && !(it.read & bw);
+            ok = ok && popcount64(tile | it.need) <= width && nsteps < WIDE_MAX_STEPS &&
+                 consts + it.consts <= WIDE_MAX_CONSTS;
+            // controls of moves that lie outside the tile (so far)
+            const uint64_t ctl = it.kind == WideItem::MOVE ? it.read : 0;
+            ok = ok && popcount64((outside | ctl) & ~(tile | it.need)) <= WIDE_MAX_OUTSIDE;
+            if (!ok) {
+                bw |= it.write;
+                br |= it.read;
+                continue;
+            }
+            tile |= it.need;
+            outside |= ctl;
+            consts += it.consts + (it.consts & 1);
+            ++nsteps;
+            taken.push_back(i);
+            done[i] = 1;
+        }
+        if (taken.empty()) return false;  // (a step wider than the tile)
+        for (int b = 0; b < n && popcount64(tile) < width; ++b) tile |= 1ull << b;
+        WidePass w;
+        w.mask = tile;
+        std::vector<char> placed(taken.size(), 0);
+        size_t todo = taken.size();
+        const int regs = std::min(opt.wide_regs, popcount64(tile));
+        for (;;) {
+            std::vector<WideMove> moves;
+            uint64_t rw = 0, rr = 0;
+            for (size_t q = 0; q < taken.size() && todo && (rw & all) != all; ++q) {
+                if (placed[q]) continue;
+                const WideItem& it = items[taken[q]];
+                if (it.kind != WideItem::MOVE || (it.write & (rw | rr)) || (it.read & rw)) {
+                    rw |= it.write;
+                    rr |= it.read;
+                    continue;
+                }
+                WideMove m;
+                m.swap = it.ws.s.type == ST_SWAP;
+                m.a = it.ws.bit[0];
+                m.b = m.swap ? it.ws.bit[1] : it.ws.s.cm ? __builtin_ctzll(it.ws.s.cm) : -1;
+                moves.push_back(m);
+                placed[q] = 1;
+                --todo;
+                --left;
+            }
+            if (!todo || (int)w.rounds.size() == WIDE_MAX_ROUNDS) {
+                w.moves = std::move(moves);
+                break;
+            }
+            // the next round: what its first step decides (rotations, then other steps on their
+            // bits, or pair blocks alone)
+            WideRound r;
+            r.moves = std::move(moves);
+            uint64_t bits = 0, fixed = 0;  // fixed: bits whose rotation is complete
+            bool only_pairs = false, any = false;
+            int order[4], nb = 0, npair = 0;
+            auto reg = [&](int b) {
+                for (int m = 0; m < nb; ++m)
+                    if (order[m] == b) return m;
+                order[nb] = b;
+                return nb++;
+            };
+            rw = rr = 0;
+            for (size_t q = 0; q < taken.size() && (rw & all) != all; ++q) {
+                if (placed[q]) continue;
+                const WideItem& it = items[taken[q]];
+                bool ok = it.kind != WideItem::MOVE && !(it.write & (rw | rr)) && !(it.read & rw) &&
+                          popcount64(bits | it.need) <= regs;
+                if (ok && any) ok = (it.kind == WideItem::PAIR) == only_pairs;
+                if (ok && it.kind == WideItem::PAIR)
+                    ok = npair < (regs >= 4 ? 2 : 1) && !(bits & it.need);
+                // a rotation after other steps of the round that reach its bit waits
+                if (ok && (it.kind == WideItem::PRE || it.kind == WideItem::ROT)) {
+                    const int b = it.ws.bit[0];
+                    int m = -1;
+                    for (int k = 0; k < nb; ++k)
+                        if (order[k] == b) m = k;
+                    if (fixed & it.need) ok = false;
+                    else if (m >= 0 && it.kind == WideItem::ROT) ok = !r.has_rot[m] && !r.has_post[m];
+                    else if (m >= 0) ok = r.has_rot[m] ? !r.has_post[m] : !r.has_pre[m];
+                }
+                if (!ok) {
+                    rw |= it.write;
+                    rr |= it.read;
+                    continue;
+                }
+                any = true;
+                only_pairs = it.kind == WideItem::PAIR;
+                bits |= it.need;
+                switch (it.kind) {
+                    case WideItem::PAIR: {
+                        const int hi = std::max(it.ws.bit[0], it.ws.bit[1]);
+                        const int lo = std::min(it.ws.bit[0], it.ws.bit[1]);
+                        reg(lo);
+                        reg(hi);
+                        r.pairs[npair] = it.ws;
+                        r.has_pair[npair++] = true;
+                        break;
+                    }
+                    case WideItem::ROT: {
+                        const int m = reg(it.ws.bit[0]);
+                        r.rot[m] = it.ws;
+                        r.has_rot[m] = true;
+                        break;
+                    }
+                    case WideItem::PRE: {
+                        const int m = reg(it.ws.bit[0]);
+                        if (r.has_rot[m]) {
+                            r.post[m] = it.ws;
+                            r.has_post[m] = true;
+                        } else {
+                            r.pre[m] = it.ws;
+                            r.has_pre[m] = true;
+                        }
+                        break;
+                    }
+                    default:
+                        for (int k = 0; k < 2; ++k)
+                            if (it.ws.bit[k] >= 0) reg(it.ws.bit[k]);
+                        fixed |= it.write | it.read;
+                        r.steps.push_back(it.ws);
+                }
+                placed[q] = 1;
+                --todo;
+                --left;
+            }
+            if (!any) return false;  // (a step on more bits than a round holds)
+            r.nbits = nb;
+            for (int m = 0; m < nb; ++m) r.bits[m] = order[m];
+            w.rounds.push_back(std::move(r));
+        }
+        // steps past the last round wait for the next pass (every step placed commutes with them)
+        for (size_t q = 0; q < taken.size(); ++q)
+            if (!placed[q]) {
+                done[taken[q]] = 0;
+                first = std::min(first, taken[q]);
+            }
+        out->push_back(std::move(w));
+    }
+    return true;
+}
+
+}  // namespace
+
 int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size_t n_mats,
                const uint8_t* none, size_t n_none, const PlanOptions& opt, Plan* plan) {
     plan->passes.clear();
+    plan->wides.clear();
     plan->pairs.clear();
     plan->customs.clear();
     plan->table_ff.clear();
@@ -1132,7 +1429,8 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
                h.need[0] >= 0;
     };
     auto is_sw = [&](size_t i) { return block_at[i] < 0 && steps[i].s.type == ST_SWAP; };
-    for (size_t i = 0; i < steps.size(); ++i) {
+    auto emit_tiles = [&](size_t begin, size_t end) {
+    for (size_t i = begin; i < end; ++i) {
         if (block_at[i] >= 0) {
             flush();
             Pass p;
@@ -1144,7 +1442,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
             // longest run of controlled-X / swap steps forming one involution
             uint64_t targets = 0, controls = 0, swapped = 0;
             size_t j = i;
-            while (j < steps.size() && (is_cx(j) || is_sw(j))) {
+            while (j < end && (is_cx(j) || is_sw(j))) {
                 if (is_sw(j)) {
                     const uint64_t sb = (1ull << steps[j].need[0]) | (1ull << steps[j].need[1]);
                     if (sb & (targets | controls | swapped)) break;
@@ -1249,6 +1547,127 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
         cur_steps.push_back(h);
     }
     flush();
+    };
+    // Segments: Custom blocks, runs of pair blocks kept for the pair passes, runs of swaps (one
+    // index permutation) and, between them, what wide passes may take.
+    auto emit_segment = [&](size_t begin, size_t end) {
+        if (begin >= end) return;
+        const size_t before = plan->passes.size();
+        emit_tiles(begin, end);
+        if (opt.wide_bits <= 0) return;
+        size_t pairs = 0, tiles = 0;
+        bool arith = false;
+        for (size_t q = before; q < plan->passes.size(); ++q) {
+            const Pass& p = plan->passes[q];
+            (p.pair >= 0 ? pairs : tiles) += 1;
+            arith = arith || p.arith;
+        }
+        tiles += opt.group_pairs ? (pairs + 1) / 2 : pairs;
+        if (!arith || tiles < 2) return;
+        // Large float-pair registers: cycles per amplitude and SM. A tile pass runs at the larger of
+        // its memory time (1.4; half that in the L2 cache) and its arithmetic (46 packed operations a
+        // cycle, pair blocks 54); a wide pass's arithmetic runs at 36 a cycle, plus 0.4 for its loads
+        // and stores; either takes 5 us to launch and drain. (Measured, tile against wide passes: 24
+        // qubits, ansatz layers (dense 2x2s) 6.29 / 5.3 ms, random columns (mostly pair blocks) 5.46 /
+        // 5.62 ms; 20 qubits, 40 random columns 0.58 / 0.39 ms, 20 brickwork layers 0.95 / 0.98 ms.)
+        const bool by_time = opt.policy == POL_FF && n >= opt.wide_large_qubits;
+        const double launch = 5e-6 * 152 * 1.9e9 / std::ldexp(1.0, n);
+        double tile_time = 0.0;
+        auto step_ops = [](const DevStep& d, double dense) {
+            const double part = std::ldexp(1.0, -std::min(popcount64(d.cm), 8));
+            switch (d.type) {
+                case ST_DENSE: return dense * part;
+                case ST_REAL: return 19.0 * part;
+                case ST_PHASE:
+                case ST_DIAG: return d.unit ? 1.0 : 19.0 * part;
+                case ST_TABLE: return 19.0 * d.nfields * part;
+                case ST_DENSE4: return 91.0;
+                default: return 1.0;
+            }
+        };
+        if (by_time) {
+            const double memory = n <= 22 ? 0.7 : 1.4;
+            size_t odd = 0;
+            for (size_t q = before; q < plan->passes.size(); ++q) {
+                const Pass& p = plan->passes[q];
+                double cycles = 0.0;
+                for (const DevStep& d : p.steps) cycles += step_ops(d, 43.0) / 46.0;
+                if (p.pair >= 0) {
+                    if (opt.group_pairs && odd++ % 2) continue;  // (two blocks a pass)
+                    cycles = (opt.group_pairs ? 182.0 : 91.0) / 54.0;
+                }
+                tile_time += launch + std::max(p.arith ? memory : memory * p.touched, cycles);
+            }
+            // before any scheduling: a dense 2x2 as a real one and one phase at best
+            double least = 0.0;
+            for (size_t q = begin; q < end; ++q) least += step_ops(steps[q].s, 31.5);
+            if (least / 36.0 > tile_time) return;
+        }
+        std::vector<WidePass> wide;
+        if (!wide_schedule(steps, begin, end, n, opt, tiles, &wide)) return;
+        if (by_time) {
+            double ops = 0.0;
+            for (const WidePass& w : wide)
+                for (const WideRound& r : w.rounds) {
+                    for (int m = 0; m < r.nbits; ++m)
+                        ops += (r.has_pre[m] ? 10.5 : 0.0) + (r.has_post[m] ? 10.5 : 0.0) +
+                               (r.has_rot[m] ? step_ops(r.rot[m].s, 43.0) + 2.0 : 0.0);
+                    ops += 91.0 * ((int)r.has_pair[0] + (int)r.has_pair[1]);
+                    for (const WideStep& d : r.steps) ops += 8.0 + step_ops(d.s, 43.0);
+                }
+            if (ops / 36.0 + (0.4 + launch) * wide.size() > tile_time) return;
+        }
+        plan->passes.resize(before);
+        for (size_t q = 0; q < wide.size(); ++q) {
+            Pass p;
+            p.wide = (int)plan->wides.size();
+            p.arith = true;
+            plan->wides.push_back(std::move(wide[q]));
+            plan->passes.push_back(p);
+        }
+    };
+    size_t seg = 0, i = 0;
+    while (i < steps.size()) {
+        size_t j = i + 1;  // end of a run that is not a segment's
+        bool own = block_at[i] >= 0;
+        if (!own && opt.wide_bits > 0 && opt.wide_pairs > 0 && steps[i].s.type == ST_DENSE4) {
+            int count = 0;
+            for (size_t q = i; q < steps.size() && block_at[q] < 0 &&
+                               (steps[q].s.type == ST_DENSE4 || is_cx(q) || is_sw(q)); ++q)
+                if (steps[q].s.type == ST_DENSE4) {
+                    ++count;
+                    j = q + 1;
+                }
+            own = count >= opt.wide_pairs;
+        }
+        if (!own && opt.wide_bits > 0 && n > opt.wide_bits && is_sw(i)) {
+            size_t q = i;
+            while (q < steps.size() && is_sw(q)) ++q;
+            own = q - i >= 3;
+            j = q;
+        }
+        if (!own && opt.wide_bits > 0 && n >= opt.wide_table_qubits && i + 1 < steps.size() &&
+            steps[i + 1].s.type == ST_TABLE && block_at[i] < 0) {
+            // rows of a Fourier transform: at least four tables at most two steps apart
+            int count = 0;
+            size_t last = i;
+            for (size_t q = i + 1; q < steps.size() && q <= last + 3 + (count == 0) && block_at[q] < 0; ++q)
+                if (steps[q].s.type == ST_TABLE) {
+                    ++count;
+                    last = q;
+                }
+            own = count >= 4;
+            if (own) j = last + 1;
+        }
+        if (!own) {
+            ++i;
+            continue;
+        }
+        emit_segment(seg, i);
+        emit_tiles(i, j);
+        seg = i = j;
+    }
+    emit_segment(seg, steps.size());
     if (opt.pair_fusion && opt.group_pairs) group_pair_passes(plan);
     return QGPU_OK;
 }
@@ -1400,9 +1819,10 @@ PauliFrame pauli_frame(PauliRun* run) {
         f.s = 1.0;
         f.rho1 = unit(-m[1] / m[2]);
     } else {
-        f.rho1 = unit(-m[1] / unit(m[0]));
-        f.rho2 = unit(m[2] / unit(m[0]));
-        if (f.rho2.real() < 0.0) {  // the sign of s that leaves rho2 near 1 (Ry next to Rz: 1)
+        f.rho1 = unit(-m[1] * std::conj(m[0]));  // (one product: real for Ry next to Rz)
+        f.rho2 = unit(m[2] * std::conj(m[0]));
+        if (std::abs(f.rho1 + 1.0) <= 4.5e-16 || std::abs(f.rho2 + 1.0) <= 4.5e-16) {
+            // the sign of s that leaves one diagonal out (Ry before or after Rz)
             f.s = -f.s;
             f.rho1 = -f.rho1;
             f.rho2 = -f.rho2;

@@ -156,6 +156,7 @@ struct Pass {
     // term's bits lie in the tile, so each thread permutes only its own 16 amplitudes)
     int pair2 = -1;
     std::vector<XTerm> pre, post;
+    int wide = -1;                     // >= 0: this pass is wide pass `wide` (k_wide)
 };
 
 // A 4x4 block over full-index bits hi > lo, local index l = 2 * bit(hi) + bit(lo).
@@ -167,8 +168,41 @@ struct PairBlock {
     uint64_t pk[128];
 };
 
+// A wide pass: steps on the bits of one tile (`mask`), in rounds of a few bits each; the kernel
+// holds the tile in shared memory and a round's bits in registers (wide.cuh). X, CNot and Swap on
+// tile bits move no data: before a round its `moves` change where each index of the tile lies.
+constexpr int MAX_WIDE_BITS = 12;
+struct WideStep {
+    DevStep s;
+    int bit[2] = {-1, -1};  // full-index bits the step acts on (DIAG: its selecting bit)
+    int pair = -1;          // ST_DENSE4: pair block
+};
+struct WideMove {
+    bool swap = false;      // exchange bits a and b; otherwise flip bit a where bit b is 1 (b < 0:
+    int a = -1, b = -1;     // always; b may lie outside the tile)
+};
+// A round applies, in this order: per register bit at most one rotation (a phase on bit value 1,
+// a 2x2, another such phase; each may be absent), pair blocks on its bits (0, 1) and (2, 3), and
+// any other steps.
+struct WideRound {
+    int nbits = 0;
+    int bits[4];
+    std::vector<WideMove> moves;
+    WideStep pre[4], rot[4], post[4];
+    bool has_pre[4] = {}, has_rot[4] = {}, has_post[4] = {};
+    WideStep pairs[2];
+    bool has_pair[2] = {};
+    std::vector<WideStep> steps;
+};
+struct WidePass {
+    uint64_t mask = 0;
+    std::vector<WideRound> rounds;
+    std::vector<WideMove> moves;  // after the last round
+};
+
 struct Plan {
     std::vector<Pass> passes;
+    std::vector<WidePass> wides;
     std::vector<PairBlock> pairs;      // fused pair blocks
     std::vector<LocalGate> customs;    // Custom gates, run by the group kernel
     std::vector<float> table_ff;       // TABLE entries as float pairs (4 floats each)
@@ -188,7 +222,16 @@ struct PlanOptions {
     bool pair_fusion = false;          // fuse gates on two wires into 4x4 blocks where cheaper
     int table_bits = 10;               // width of a phase-table field (<= MAX_TABLE_BITS)
     bool group_pairs = true;           // with pair_fusion: two pair blocks per pass, XOR terms folded in
+    // Wide passes of up to wide_bits tile bits (0: none), wide_regs bits per round, holding the
+    // wide_low lowest index bits, where they take fewer passes than the register tiles. Runs of at
+    // least wide_pairs pair blocks (0: none) stay with the pair passes (the digit passes).
+    int wide_bits = 0, wide_regs = 2, wide_low = 3, wide_pairs = 0;
+    int wide_large_qubits = 20;        // from this size the passes' times decide (float pairs)
+    int wide_table_qubits = 20;        // from this size rows of phase tables stay with tile passes
 };
+// Limits of one wide pass (its program lies in shared memory).
+constexpr int WIDE_MAX_STEPS = 128, WIDE_MAX_ROUNDS = 48, WIDE_MAX_CONSTS = 2560;
+constexpr int WIDE_MAX_OUTSIDE = 12;  // distinct controls of moves outside the tile
 
 // Elementary terms of an XOR pass, and the pass rebuilt from a subset of them (false when the
 // terms need more than MAX_XOR_TERMS entries).

@@ -537,6 +537,10 @@ __global__ void __launch_bounds__(256) k_pair(typename P::S* __restrict__ st,
     }
 }
 
+}  // namespace qgpu
+#include "wide.cuh"
+namespace qgpu {
+
 template <class P>
 struct IsArith { static constexpr bool value = true; };
 template <class T>
@@ -1291,6 +1295,16 @@ static int launch_pair(qgpu_handle* h, const PairBlock& pb, int lay) {
     return QGPU_OK;
 }
 
+static int launch_wide(qgpu_handle* h, const WideParams& p, int lay) {
+    if (h->precision == QGPU_C64) return launch_wide_pol<WideF32, PolPackedF32>(h, p);
+    switch (lay) {
+        case LAY_RES: return launch_wide_pol<WideFF, PolFFR>(h, p);
+        case LAY_IN: return launch_wide_pol<WideFF, PolFFIn>(h, p);
+        case LAY_OUT: return launch_wide_pol<WideFF, PolFFOut>(h, p);
+        default: return launch_wide_pol<WideFF, PolFF>(h, p);
+    }
+}
+
 // ---- double pair passes: two 4x4 blocks on disjoint bit pairs of a 4-bit tile --------------
 // A tile is 16 amplitudes (full indices base | combinations of the 4 bits). Its amplitudes are
 // gathered through the slot permutation of the XOR terms folded before the blocks, block A (the
@@ -1659,7 +1673,8 @@ static bool plan_resident(const qgpu_handle* h, const Plan& plan, const std::vec
     int arith = 0;
     for (size_t i = 0; i < plan.passes.size(); ++i) {
         const Pass& ps = plan.passes[i];
-        arith += (!dig[i] && ps.custom < 0 && !ps.xor_pass && ps.arith);
+        // (a wide pass holds the work of several)
+        arith += (!dig[i] && ps.custom < 0 && !ps.xor_pass && ps.arith) ? (ps.wide >= 0 ? 4 : 1) : 0;
     }
     return arith >= 8;
 }
@@ -1726,10 +1741,31 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
     const size_t nent = plan.table_f64.size() / 2;
     const float4* tab_ff = nullptr;
     const double2* tab_f64 = nullptr;
-    if (nent) {
-        const size_t ffb = align_up(nent * 16, 256);
-        int st = h->tables.ensure(ffb + nent * 16);
+    // the wide passes' programs lie behind the tables
+    std::vector<WideParams> wide(plan.wides.size());
+    std::vector<uint8_t> wide_prog;
+    std::vector<size_t> wide_at(plan.wides.size());
+    double wide_drift = 0.0;
+    for (size_t i = 0; i < plan.wides.size(); ++i) {
+        wide_at[i] = wide_prog.size();
+        if (pol == POL_F32) wide_fill<WideF32>(plan, plan.wides[i], h->n_qubits, h->dim, &wide[i], &wide_prog, &wide_drift);
+        else wide_fill<WideFF>(plan, plan.wides[i], h->n_qubits, h->dim, &wide[i], &wide_prog, &wide_drift);
+    }
+    const size_t ffb = align_up(nent * 16, 256);
+    const size_t prog_at = align_up(ffb + nent * 16, 256);
+    if (nent || !wide_prog.empty()) {
+        int st = h->tables.ensure(prog_at + wide_prog.size());
         if (st != QGPU_OK) return st;
+    }
+    if (!wide_prog.empty()) {
+        uint8_t* at = (uint8_t*)h->tables.ptr + prog_at;
+        QGPU_CUDA(copy_async(h, at, wide_prog.data(), wide_prog.size(), cudaMemcpyHostToDevice));
+        for (size_t i = 0; i < wide.size(); ++i) {
+            wide[i].prog = (const uint4*)(at + wide_at[i]);
+            wide[i].tab_ff = (const float4*)h->tables.ptr;
+        }
+    }
+    if (nent) {
         QGPU_CUDA(copy_async(h, h->tables.ptr, plan.table_ff.data(), nent * 16,
                              cudaMemcpyHostToDevice));
         QGPU_CUDA(copy_async(h, (uint8_t*)h->tables.ptr + ffb, plan.table_f64.data(), nent * 16,
@@ -1764,7 +1800,8 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
     // elsewhere a k_ff_layout pass converts. Digit runs are bracketed by k_dg_from / k_dg_to.
     static const int fuse = env_int("QGPU_FUSE_LAYOUT", 1);  // tuning knob: 0 = separate passes
     auto fusable = [](const Pass& p) {
-        return p.custom < 0 && !p.xor_pass && (p.pair >= 0 || (p.arith && p.nbits <= MAX_TILE_BITS));
+        return p.custom < 0 && !p.xor_pass &&
+               (p.pair >= 0 || p.wide >= 0 || (p.arith && p.nbits <= MAX_TILE_BITS));
     };
     int last_nonxor = (int)np - 1;
     while (last_nonxor >= 0 && plan.passes[last_nonxor].xor_pass) --last_nonxor;
@@ -1874,6 +1911,8 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
                                                                                                  : "k_dg_to");
             } else if (play == LAY_DIG && !ps->xor_pass) {
                 prof_names.push_back("k_dg2");
+            } else if (ps->wide >= 0) {
+                prof_names.push_back(std::string("k_wide<") + (resident ? "ffr" : pol_name[pol]) + ">");
             } else if (ps->pair2 >= 0) {
                 prof_names.push_back(h->precision == QGPU_C64 ? "k_pair2<f32>"
                                      : (play == LAY_RES && pair2_tc_enabled() && pair2_tc_supported(h))
@@ -1909,6 +1948,8 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
             const DgPass& d = dgp[it.pass];
             st = dg_launch_pass(h, d.bits, d.bimg.data(),
                                 reinterpret_cast<const int32_t(*)[dg::KAP]>(d.kap.data()));
+        } else if (ps->wide >= 0) {
+            st = launch_wide(h, wide[ps->wide], play);
         } else if (ps->pair2 >= 0) {
             st = launch_pair2(h, plan, *ps, play);
         } else if (ps->pair >= 0) {
@@ -1997,6 +2038,19 @@ PlanOptions plan_options_for(const qgpu_handle* h) {
     // phase-table field width (tuning knob QGPU_TABLE_BITS): 10 bits measured best on GB300 for
     // the 30-qubit QFT rows (1114 ms per step; 11: 1118, 12: 1156, 9: 1182 ms)
     o.table_bits = env_int("QGPU_TABLE_BITS", 10);
+    // wide passes (k_wide): float pairs and complex64; QGPU_WIDE=0 (read per call): off. Where the
+    // digit passes run, runs of pair blocks stay with them.
+    const char* wide = std::getenv("QGPU_WIDE");
+    if (o.policy != POL_F64 && !(wide && wide[0] == '0') && !pair2_tc_enabled()) {
+        const bool ff = o.policy == POL_FF;
+        o.wide_bits = ff ? WideFF::TBITS + WideFF::RBITS : WideF32::TBITS + WideF32::RBITS;
+        o.wide_regs = ff ? WideFF::R : WideF32::R;
+        o.wide_low = ff ? 2 : 3;
+        o.wide_pairs = ff && dg_supported(h) ? 6 : 0;
+        // (Fourier transforms, wide against tile passes: complex128 at 19 qubits 205 / 243 us, at 20
+        // 378 / 317; complex64 at 18 qubits 216 / 166 us)
+        o.wide_table_qubits = ff ? 20 : 14;
+    }
     return o;
 }
 
