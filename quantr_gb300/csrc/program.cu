@@ -2054,6 +2054,10 @@ PlanOptions plan_options_for(const qgpu_handle* h) {
     return o;
 }
 
+// exact.cu: the leading standard gates of an exact-mode program in tile passes (at: the gates' ops)
+int exact_passes(qgpu_handle* h, const qgpu_op* ops, const std::vector<LocalGate>& gates,
+                 const std::vector<size_t>& at, size_t* taken);
+
 int apply_blocks(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const double* mats,
                  size_t n_mats, const uint8_t* none, size_t n_none, int bq, int mg);  // blocks.cu
 
@@ -2101,21 +2105,42 @@ extern "C" int qgpu_apply_program(qgpu_handle* h, const qgpu_op* ops, size_t n_o
     // the exact and dense-block paths do not carry the amplitude bound through Custom gates
     bool has_custom = false;
     for (size_t g = 0; g < n_ops; ++g) has_custom = has_custom || ops[g].kind == QGPU_GATE_CUSTOM;
+    const double bound_before = h->norm_valid ? h->norm_bound : -1.0;
     if (has_custom && ((h->precision == QGPU_C128 && h->mode == QGPU_MODE_EXACT) || h->block_qubits > 0))
         h->norm_valid = false;
     if (h->precision == QGPU_C128 && h->mode == QGPU_MODE_EXACT) {
         std::vector<LocalGate> gates;
+        std::vector<size_t> at;
         gates.reserve(n_ops);
+        at.reserve(n_ops);
         for (size_t g = 0; g < n_ops; ++g) {
             if (ops[g].kind == QGPU_GATE_ID) continue;  // simulation.rs:38-41
             LocalGate lg;
             int st = tabulate(ops[g], h->n_qubits, mats, n_mat_doubles, none_flags, n_none_flags, &lg);
             if (st != QGPU_OK) return st;
             gates.push_back(std::move(lg));
+            at.push_back(g);
+        }
+        // Tile passes leave out products with 0 and 1, which on finite amplitudes changes no value:
+        // they take the gates up to the first Custom one when the register's norm is known or found
+        // to be finite and far from overflow. The rest goes through one launch per gate.
+        size_t taken = 0;
+        if (!gates.empty() && ops[at[0]].kind != QGPU_GATE_CUSTOM) {
+            double bound = bound_before;
+            if (!(bound >= 0.0)) {
+                double2 r;
+                int st = reduce_state(h, 0, &r);
+                if (st != QGPU_OK) return st;
+                bound = std::sqrt(r.x);
+            }
+            if (bound < 1e100) {
+                int st = exact_passes(h, ops, gates, at, &taken);
+                if (st != QGPU_OK) return st;
+            }
         }
         // tables for a window of gates at a time keeps the device staging bounded
         const size_t window = 512;
-        for (size_t i = 0; i < gates.size(); i += window) {
+        for (size_t i = taken; i < gates.size(); i += window) {
             std::vector<const LocalGate*> part;
             for (size_t j = i; j < gates.size() && j < i + window; ++j) part.push_back(&gates[j]);
             int st = run_groups(h, part);
