@@ -312,7 +312,7 @@ def run_batch_leg(args) -> None:
     one qgpu_batch_run call per rank. Under torchrun the circuits shard across ranks by cost
     (batch.shard) and the results come back with one all-reduce of flat arrays; the time is the
     slowest rank's, between barriers. Reports circuits/s and, per size, the fusion budget and
-    adjoint sweep form the autotuner picked."""
+    adjoint sweep form used."""
     import torch
 
     from quantr_gb300 import _native as nat

@@ -59,7 +59,7 @@ def batch_config(count: int = 4096, seed: int = 5, layers: int = 4, n_min: int =
 
 def run_batch(circuits: list[BatchCircuit], precision: int = nat.QGPU_C128):
     """Energies [len], per-circuit gradient arrays (one entry per op) and, per qubit count of
-    the register-pass circuits, the autotuner's picks, all on the current GPU."""
+    the register-pass circuits, the fusion budget and sweep form used, all on the current GPU."""
     lib = nat.lib()
     items = (QgpuBatchItem * max(1, len(circuits)))()
     ops, obs = [], []
@@ -90,8 +90,8 @@ def run_batch(circuits: list[BatchCircuit], precision: int = nat.QGPU_C128):
     out_g = []
     for i, c in enumerate(circuits):
         out_g.append(grads[items[i].grad_offset: items[i].grad_offset + len(c.program.ops)].copy())
-    # per size: the fusion budget (float-pair for complex128, f32 for complex64) and the adjoint
-    # sweep form the autotuner picked
+    # per size: the fusion budget (float-pair for complex128, f32 for complex64) and the form of the
+    # adjoint sweep
     picks = {q: {"fusion_budget": tuned[q] & 0xFFFF,
                  "adjoint_sweep": "grouped" if tuned[q] >> 16 else "per-wire"}
              for q in range(41) if tuned[q]}

@@ -1804,13 +1804,22 @@ qgpu_op inverse_op(const qgpu_op& op) {
 PauliFrame pauli_frame(PauliRun* run) {
     const std::array<cd, 4>& m = run->undo;  // m00 m01 m10 m11
     PauliFrame f;
-    f.c = std::abs(m[0]);
-    f.s = std::abs(m[1]);
-    const double r = std::hypot(f.c, f.s);
-    f.c /= r;
-    f.s /= r;
     auto unit = [](cd z) { return z / std::abs(z); };
-    if (m[1] == cd(0.0, 0.0)) {  // diagonal
+    if (!run->framed) {
+        f.c = std::abs(m[0]);
+        f.s = std::abs(m[1]);
+        const double r = std::hypot(f.c, f.s);
+        f.c /= r;
+        f.s /= r;
+    }
+    if (run->framed) {
+        f = run->frame;
+        if (f.s == 0.0) {  // diagonal
+            f.rho1 *= f.rho2;
+            f.rho2 = 1.0;
+            if (f.c < 0.0) f.c = 1.0;
+        }
+    } else if (m[1] == cd(0.0, 0.0)) {  // diagonal
         f.c = 1.0;
         f.s = 0.0;
         f.rho1 = unit(m[3] / m[0]);
@@ -1821,12 +1830,13 @@ PauliFrame pauli_frame(PauliRun* run) {
     } else {
         f.rho1 = unit(-m[1] * std::conj(m[0]));  // (one product: real for Ry next to Rz)
         f.rho2 = unit(m[2] * std::conj(m[0]));
-        if (std::abs(f.rho1 + 1.0) <= 4.5e-16 || std::abs(f.rho2 + 1.0) <= 4.5e-16) {
-            // the sign of s that leaves one diagonal out (Ry before or after Rz)
-            f.s = -f.s;
-            f.rho1 = -f.rho1;
-            f.rho2 = -f.rho2;
-        }
+    }
+    if (f.c != 0.0 && f.s != 0.0 &&
+        (std::abs(f.rho1 + 1.0) <= 4.5e-16 || std::abs(f.rho2 + 1.0) <= 4.5e-16)) {
+        // the sign of s that leaves one diagonal out (Ry before or after Rz)
+        f.s = -f.s;
+        f.rho1 = -f.rho1;
+        f.rho2 = -f.rho2;
     }
     if (std::abs(f.rho1 - 1.0) <= 4.5e-16) f.rho1 = 1.0;
     if (std::abs(f.rho2 - 1.0) <= 4.5e-16) f.rho2 = 1.0;
@@ -1871,18 +1881,12 @@ std::vector<std::pair<uint64_t, std::vector<size_t>>> adj_group_passes(const std
 
 int pauli_run(const qgpu_op* ops, const std::vector<size_t>& gw, int n, PauliRun* out) {
     const size_t k = gw.size();
-    std::vector<std::array<cd, 4>> fwd(k), inv(k);  // row-major 2x2: m[2 l + j]
-    for (size_t q = 0; q < k; ++q) {
-        LocalGate a, b;
-        int st = tabulate(ops[gw[q]], n, nullptr, 0, nullptr, 0, &a);
-        if (st == QGPU_OK) st = tabulate(inverse_op(ops[gw[q]]), n, nullptr, 0, nullptr, 0, &b);
-        if (st != QGPU_OK) return st;
-        for (int l = 0; l < 2; ++l)
-            for (int j = 0; j < 2; ++j) {
-                fwd[q][2 * l + j] = a.M[j * 2 + l];
-                inv[q][2 * l + j] = b.M[j * 2 + l];
-            }
-    }
+    // a single-wire gate, row-major: m[2 l + j] (column j its image of |j>)
+    auto matrix = [](const qgpu_op& op) {
+        cd c0[2], c1[2];
+        one_qubit_images(op, c0, c1);
+        return std::array<cd, 4>{c0[0], c1[0], c0[1], c1[1]};
+    };
     auto mul = [](const std::array<cd, 4>& x, const std::array<cd, 4>& y) {
         return std::array<cd, 4>{x[0] * y[0] + x[1] * y[2], x[0] * y[1] + x[1] * y[3],
                                  x[2] * y[0] + x[3] * y[2], x[2] * y[1] + x[3] * y[3]};
@@ -1891,9 +1895,39 @@ int pauli_run(const qgpu_op* ops, const std::vector<size_t>& gw, int n, PauliRun
     std::array<cd, 4> undo{cd(1), cd(0), cd(0), cd(1)}, V{cd(1), cd(0), cd(0), cd(1)};
     out->rots.clear();
     for (int m = 0; m < 5; ++m) out->need[m] = false;
+    // diagonals, real rotations, diagonals: the frame is read off the gates
+    bool turned = false, between = false;
+    out->framed = true;
+    out->frame = PauliFrame();
+    PauliFrame& f = out->frame;
     for (size_t q = 0; q < k; ++q) {  // q = 0 is the last gate of the run
-        undo = mul(inv[q], undo);
         const qgpu_op& op = ops[gw[q]];
+        int arity = 0;
+        const int st = op_arity(op, n, &arity);
+        if (st != QGPU_OK) return st;
+        const std::array<cd, 4> inv = matrix(inverse_op(op));
+        undo = mul(inv, undo);
+        switch (op.kind) {
+            case QGPU_GATE_Z: case QGPU_GATE_S: case QGPU_GATE_SDAG: case QGPU_GATE_T: case QGPU_GATE_TDAG:
+            case QGPU_GATE_RZ: case QGPU_GATE_PHASE: {
+                if (op.kind == QGPU_GATE_PHASE) break;  // (a global phase)
+                const cd r = op.kind == QGPU_GATE_RZ ? cd(std::cos(op.param), -std::sin(op.param)) : inv[3];
+                cd& rho = turned ? f.rho2 : f.rho1;
+                rho = rho == cd(1.0, 0.0) ? r : rho * r;
+                between = turned;
+                break;
+            }
+            case QGPU_GATE_RY: case QGPU_GATE_Y90: case QGPU_GATE_MY90: {
+                const double c = inv[0].real(), s = inv[2].real();
+                const PauliFrame g = f;
+                f.c = turned ? c * g.c - s * g.s : c;
+                f.s = turned ? s * g.c + c * g.s : s;
+                out->framed = out->framed && !between;
+                turned = true;
+                break;
+            }
+            default: out->framed = false;
+        }
         if (is_rotation(op.kind)) {
             std::array<cd, 4> P{cd(0), cd(0), cd(0), cd(0)};
             switch (op.kind) {
@@ -1913,17 +1947,15 @@ int pauli_run(const qgpu_op* ops, const std::vector<size_t>& gw, int n, PauliRun
             for (int m = 1; m <= 4; ++m) out->need[m] = out->need[m] || c[m] != 0.0;
             out->rots.emplace_back(gw[q], c);
         }
-        V = mul(V, fwd[q]);  // the gates after the next one back
+        if (q + 1 < k) V = mul(V, matrix(op));  // the gates after the next one back
     }
     out->undo = undo;
     return QGPU_OK;
 }
 
-// Whether ops (applied in order) form an affine index map; if so, the gather tables of its
-// inverse: tabs[c * 256 + v] = xor of the inverse map's columns for the set bits of v (bits
-// 8c .. 8c+7), *d = inverse map of 0.
-bool affine_tables(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t>* tabs,
-                   uint64_t* d) {
+// Whether ops (applied in order) form an affine index map; if so, the columns of its inverse, *d =
+// inverse map of 0.
+bool affine_columns(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t>* col, uint64_t* d) {
     for (size_t g = 0; g < n_ops; ++g) {
         const int k = ops[g].kind;
         if (k != QGPU_GATE_CNOT && k != QGPU_GATE_X && k != QGPU_GATE_SWAP) return false;
@@ -1947,8 +1979,15 @@ bool affine_tables(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t
         return y;
     };
     *d = inv(0);
-    std::vector<uint64_t> col(n);
-    for (int b = 0; b < n; ++b) col[b] = inv(1ull << b) ^ *d;
+    col->resize(n);
+    for (int b = 0; b < n; ++b) (*col)[b] = inv(1ull << b) ^ *d;
+    return true;
+}
+
+bool affine_tables(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t>* tabs,
+                   uint64_t* d) {
+    std::vector<uint64_t> col;
+    if (!affine_columns(ops, n_ops, n, &col, d)) return false;
     const int nchunks = (n + 7) / 8;
     tabs->assign((size_t)nchunks * 256, 0);
     for (int c = 0; c < nchunks; ++c)

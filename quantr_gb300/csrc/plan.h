@@ -39,6 +39,16 @@ bool is_rotation(int kind);
 // The inverse of a non-Custom op as another op (U^dagger), quantr's conventions.
 qgpu_op inverse_op(const qgpu_op& op);
 
+// The undo of a run, undo = e^{i a} diag(1, rho2) [[c, -s], [s, c]] diag(1, rho1): the phase e^{i a}
+// (common to both vectors of a sweep) is dropped. Conjugating by diag(1, rho1) mixes X and Y only,
+// so a rotation's coefficients are turned into those of the sums taken after it: for a run that
+// ends in Ry, Rz or Rz alone no X sum is left. Coefficients up to 4.5e-16 in magnitude (the
+// rounding of the products they come from) are dropped.
+struct PauliFrame {
+    double c = 1.0, s = 0.0;
+    cd rho1 = 1.0, rho2 = 1.0;
+};
+
 // A run of single-wire gates on one wire undone by the adjoint sweep in one pass. A rotation
 // G = exp(-i theta P / 2) followed on its wire by V (the run's later gates) has gradient
 // Im <lambda| V P V^dag |phi>, taken before the run is undone; V P V^dag = q0 I + qx X + qy Y + qz Z
@@ -49,19 +59,13 @@ struct PauliRun {
     // per rotation: its op index and the coefficients of the sums (1 X, 2 Y, 3 Z, 4 -I)
     std::vector<std::pair<size_t, std::array<double, 5>>> rots;
     bool need[5] = {false, false, false, false, false};  // sums with a non-zero coefficient
+    // For a run of diagonal gates, real rotations and diagonal gates: the frame from the gates' own
+    // angles, each constant rounded once (from `undo` it takes the rounding of the products).
+    bool framed = false;
+    PauliFrame frame;
 };
 // gw: the run's op indices into ops, in reverse order (gw[0] the run's last gate).
 int pauli_run(const qgpu_op* ops, const std::vector<size_t>& gw, int n, PauliRun* out);
-
-// The undo of a run, undo = e^{i a} diag(1, rho2) [[c, -s], [s, c]] diag(1, rho1): the phase e^{i a}
-// (common to both vectors of a sweep) is dropped. Conjugating by diag(1, rho1) mixes X and Y only,
-// so a rotation's coefficients are turned into those of the sums taken after it: for a run that
-// ends in Ry, Rz or Rz alone no X sum is left. Coefficients up to 4.5e-16 in magnitude (the
-// rounding of the products they come from) are dropped.
-struct PauliFrame {
-    double c = 1.0, s = 0.0;
-    cd rho1 = 1.0, rho2 = 1.0;
-};
 PauliFrame pauli_frame(PauliRun* run);
 
 // The passes of a grouped adjoint sweep (the runs of single-wire gates of many wires per pass):
@@ -78,6 +82,8 @@ std::vector<std::pair<uint64_t, std::vector<size_t>>> adj_group_passes(const std
 // h(y) = *d xor tabs[c * 256 + byte c of y] over the 8-bit chunks c of y.
 bool affine_tables(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t>* tabs,
                    uint64_t* d);
+// The same map by its columns: h(y) = *d xor col[b] over the set bits b of y.
+bool affine_columns(const qgpu_op* ops, size_t n_ops, int n, std::vector<uint64_t>* col, uint64_t* d);
 
 // ---------------------------------------------------------------------------------------------
 // Fused passes for the fast kernels (QGPU_MODE_FAST / QGPU_MODE_F64 / complex64).
