@@ -9,11 +9,13 @@
 // vector is read 1 + ceil((n - 11) / 8) times. complex128 runs in float pairs (packed Dot2), the
 // energy sum included; complex64 in f32 with the energy as error-free transformed products.
 // What bounds it: the float-pair multiply-adds (12 packed operations per amplitude and bit, ~2.1
-// cycles per amplitude and SM in an 11-bit pass, against 0.7 cycles for its HBM read); complex64:
-// the shared-memory reads (8 of 11 neighbours, 64 B per amplitude) and HBM.
+// cycles per amplitude and SM in an 11-bit pass, against 0.7 cycles for its HBM read; the energy
+// alone takes half of them, k_zzx_energy); complex64: the shared-memory reads (8 of 11 neighbours,
+// 64 B per amplitude) and HBM.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include <math_constants.h>
@@ -28,6 +30,12 @@ constexpr int ZZX_BITS = 11;    // tile bits: 8 in the thread index, 3 in a thre
 constexpr int ZZX_LOW = 3;      // low bits of the tiles of the later passes
 constexpr int ZZX_REGS = 8;     // amplitudes per thread
 constexpr int ZZX_FIELD = ZZX_BITS - ZZX_LOW;
+// Smallest complex128 register whose energy alone is taken pair by pair (k_zzx_energy: two CTAs per
+// SM, so fewer tiles leave SMs idle): energy call, k_zzx / k_zzx_energy, at 20 qubits 72 / 85 us, at
+// 21 96 / 99, at 22 150 / 133, at 24 541 / 382.
+constexpr int ZZX_PAIRS_QUBITS = 22;
+
+constexpr u64 ZZX_SIGNS = 0x8000000080000000ull;  // both lanes negated
 
 // Coefficients as the packed operands of a Dot2 term (hi, lo, -hi, -lo), both lanes alike.
 struct ZzxCoef {
@@ -42,6 +50,7 @@ struct ZzxParams {
     // the diagonal (first pass): ZZ coefficient of bits (q, q+1) and of the wrap (0, n-1)
     float2 zz[MAX_HAM_QUBITS];
     float2 wrap;
+    double twice[ZZX_BITS];     // twice the X coefficient of tile bit m (0: not this pass's)
 };
 
 struct ZvFF {
@@ -49,6 +58,9 @@ struct ZvFF {
     using V = ffp;
     static __device__ __forceinline__ V split(S a) { return to_ffp(a); }
     // the split keeps neither magnitudes past the float range nor infinities and NaN
+    // place of a tile index in shared memory: each arrangement of k_zzx_energy reads 8 different
+    // 16-byte banks per phase
+    static __device__ __forceinline__ unsigned place(unsigned x) { return x ^ ((x >> 3) & 7u); }
     static __device__ __forceinline__ bool too_large(S a) {
         constexpr int most = (1023 + 40) << 20;
         return (__double2hiint(a.x) & 0x7FFFFFFF) >= most || (__double2hiint(a.y) & 0x7FFFFFFF) >= most;
@@ -66,8 +78,7 @@ struct ZvFF {
         }
     };
     static __device__ __forceinline__ void term(PDot2& acc, const V& a, const V& b) {
-        const u64 m = p2(-1.f, -1.f);
-        const u64 c[4] = {a.h, a.l, pmul(a.h, m), pmul(a.l, m)};
+        const u64 c[4] = {a.h, a.l, a.h ^ ZZX_SIGNS, a.l ^ ZZX_SIGNS};
         acc.add(c, b.h, b.l);
     }
     static __device__ __forceinline__ V plus(const V& a, const V& b) {
@@ -102,7 +113,7 @@ struct ZvF32 {
     // the product's rounding error and the sum's both go to the error sum, as in PDot2::add
     static __device__ __forceinline__ void term(PDot2& acc, V a, V b) {
         const u64 p = pmul(a, b);
-        const u64 rn = pfma(pmul(a, p2(-1.f, -1.f)), b, p);
+        const u64 rn = pfma(a ^ ZZX_SIGNS, b, p);
         const u64 t = padd(acc.s, p);
         const u64 bb = psub(t, acc.s);
         const u64 q = padd(psub(acc.s, psub(t, bb)), psub(p, bb));
@@ -134,113 +145,65 @@ __device__ __forceinline__ double zzx_value(const PDot2& acc) {
     return ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
 }
 
-// FIRST: the diagonal and the 11 lowest bits; otherwise the bits of p.terms (above the 3 lowest).
-// VEC: psi's copy goes to phi and H psi to lam, both in the sweep's layout (P::put); later
-// passes read phi and add to lam. Without VEC only the energy is formed. partial[blockIdx] gets the
-// pass's share of Re <psi|H psi>, and with FIRST partial[gridDim + blockIdx] that of <psi|psi>.
-template <class P, bool FIRST, bool VEC>
-__global__ void __launch_bounds__(ZZX_THREADS, sizeof(typename P::S) == 8 ? 4 : FIRST && VEC ? 2 : 3)
-k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
-      typename P::S* __restrict__ lam, const __grid_constant__ ZzxParams p,
-      double* __restrict__ partial) {
-    using V = typename P::V;
-    __shared__ __align__(16) V tile[1 << ZZX_BITS];
-    __shared__ float2 t_low[64], t_high[64], t_base[4];
-    const unsigned t = threadIdx.x;
+// Amplitude of tile index t + 256 j of tile g: base + j * step.
+template <bool FIRST>
+__device__ __forceinline__ void zzx_place(const ZzxParams& p, uint64_t g, unsigned t, uint64_t& base,
+                                          uint64_t& step) {
     if (FIRST) {
-        // the diagonal's part inside the tile: pairs of bits 0..5 and of bits 5..10
+        base = (g << ZZX_BITS) + t;
+        step = ZZX_THREADS;
+    } else {
+        const uint64_t mid = g & ((1ull << (p.shift - ZZX_LOW)) - 1ull);
+        const uint64_t top = g >> (p.shift - ZZX_LOW);
+        base = (top << (p.shift + ZZX_FIELD)) | (mid << ZZX_LOW) | (t & ((1u << ZZX_LOW) - 1u)) |
+               ((uint64_t)(t >> ZZX_LOW) << p.shift);
+        step = 1ull << (p.shift + 8 - ZZX_LOW);
+    }
+}
+
+// The diagonal in three parts: pairs of bits 0..5 and of bits 5..10 (tables by thread, once), and
+// what lies above the tile g, one lane of a warp per pair of bits, with its four combinations with
+// the pairs (10, 11) and (0, n-1) that reach into the tile.
+struct ZzxDiag {
+    float2 low[64], high[64], base[4];
+    __device__ __forceinline__ void tables(const ZzxParams& p, unsigned t) {
         if (t < 128) {
             const unsigned x = t & 63u;
             const int q0 = t < 64 ? 0 : 5;
             float2 d = make_float2(0.f, 0.f);
             for (int q = 0; q < 5; ++q) d = ff_plus(d, ff_sign(p.zz[q0 + q], (x >> q) ^ (x >> (q + 1))));
-            (t < 64 ? t_low : t_high)[x] = d;
+            (t < 64 ? low : high)[x] = d;
         }
     }
-    bool large = false;
-    PDot2 acc, nrm;
-    acc.s = acc.en = nrm.s = nrm.en = 0;
-    for (uint64_t g = blockIdx.x; g < p.ntiles; g += gridDim.x) {
-        uint64_t base, step;  // amplitude of tile index t + 256 j: base + j * step
-        if (FIRST) {
-            base = (g << ZZX_BITS) + t;
-            step = ZZX_THREADS;
-        } else {
-            const uint64_t mid = g & ((1ull << (p.shift - ZZX_LOW)) - 1ull);
-            const uint64_t top = g >> (p.shift - ZZX_LOW);
-            base = (top << (p.shift + ZZX_FIELD)) | (mid << ZZX_LOW) | (t & ((1u << ZZX_LOW) - 1u)) |
-                   ((uint64_t)(t >> ZZX_LOW) << p.shift);
-            step = 1ull << (p.shift + 8 - ZZX_LOW);
+    __device__ __forceinline__ void above(const ZzxParams& p, uint64_t g, unsigned t) {
+        if (t >= 32) return;
+        const int q = ZZX_BITS + (int)t;
+        float2 d = make_float2(0.f, 0.f);
+        if (q + 1 < p.n) d = ff_sign(p.zz[q], (unsigned)((g >> t) ^ (g >> (t + 1))));
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+            const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d.x, w),
+                                         __shfl_xor_sync(0xffffffffu, d.y, w));
+            d = ff_plus(d, o);
         }
-        V v[ZZX_REGS];
-        if constexpr (!FIRST && VEC) {
-#pragma unroll
-            for (int j = 0; j < ZZX_REGS; ++j) v[j] = P::get(phi + base + j * step);
-        } else {
-            typename P::S raw[ZZX_REGS];
-#pragma unroll
-            for (int j = 0; j < ZZX_REGS; ++j) raw[j] = psi[base + j * step];
-#pragma unroll
-            for (int j = 0; j < ZZX_REGS; ++j) {
-                v[j] = P::split(raw[j]);
-                if constexpr (FIRST) large = large || P::too_large(raw[j]);
-            }
-        }
-        __syncthreads();  // the previous tile's readers are done
-#pragma unroll
-        for (int j = 0; j < ZZX_REGS; ++j) tile[t + ZZX_THREADS * j] = v[j];
-        if (FIRST && t < 32) {
-            // the diagonal's part above the tile, one lane per pair of bits, and its four
-            // combinations with the pairs (10, 11) and (0, n-1) that reach into the tile
-            const int q = ZZX_BITS + (int)t;
-            float2 d = make_float2(0.f, 0.f);
-            if (q + 1 < p.n) d = ff_sign(p.zz[q], (unsigned)((g >> t) ^ (g >> (t + 1))));
-#pragma unroll
-            for (int w = 16; w > 0; w >>= 1) {
-                const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d.x, w),
-                                             __shfl_xor_sync(0xffffffffu, d.y, w));
-                d = ff_plus(d, o);
-            }
-            if (t < 4) {
-                d = ff_plus(d, ff_sign(p.zz[ZZX_BITS - 1], (t & 1u) ^ (unsigned)(g & 1ull)));
-                d = ff_plus(d, ff_sign(p.wrap, (t >> 1) ^ (unsigned)(g >> (p.n - 1 - ZZX_BITS))));
-                t_base[t] = d;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < ZZX_REGS; ++j) {
-            typename P::Sum s;
-            if constexpr (FIRST) {
-                float2 d = ff_plus(t_low[t & 63u], t_high[((t >> 5) & 7u) | (j << 3)]);
-                d = ff_plus(d, t_base[(j >> 2) | ((t & 1u) << 1)]);
-                const u64 c[4] = {p2(d.x, d.x), p2(d.y, d.y), p2(-d.x, -d.x), p2(-d.y, -d.y)};
-                s.first(c, v[j]);
-            } else {
-                const u64 zero[4] = {0, 0, 0, 0};
-                s.first(zero, v[j]);
-            }
-#pragma unroll
-            for (int m = FIRST ? 0 : ZZX_LOW; m < 8; ++m)
-                if ((p.terms >> m) & 1u) s.add(p.x[m].c, tile[(t ^ (1u << m)) + ZZX_THREADS * j]);
-#pragma unroll
-            for (int m = 8; m < ZZX_BITS; ++m)
-                if ((p.terms >> m) & 1u) s.add(p.x[m].c, v[j ^ (1 << (m - 8))]);
-            const V o = s.result();
-            P::term(acc, v[j], o);
-            if constexpr (FIRST) P::term(nrm, v[j], v[j]);
-            if constexpr (VEC) {
-                if constexpr (FIRST) {
-                    P::put(phi + base + j * step, v[j]);
-                    P::put(lam + base + j * step, o);
-                } else {
-                    P::put(lam + base + j * step, P::plus(P::get(lam + base + j * step), o));
-                }
-            }
+        if (t < 4) {
+            d = ff_plus(d, ff_sign(p.zz[ZZX_BITS - 1], (t & 1u) ^ (unsigned)(g & 1ull)));
+            d = ff_plus(d, ff_sign(p.wrap, (t >> 1) ^ (unsigned)(g >> (p.n - 1 - ZZX_BITS))));
+            base[t] = d;
         }
     }
-    // per-CTA sums: warp shuffles, then one value per warp
-    double e = zzx_value(acc), q = FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0;
+    // the diagonal entry of tile index t + 256 j as a Dot2 coefficient
+    __device__ __forceinline__ ZzxCoef entry(unsigned t, int j) const {
+        float2 d = ff_plus(low[t & 63u], high[((t >> 5) & 7u) | (j << 3)]);
+        d = ff_plus(d, base[(j >> 2) | ((t & 1u) << 1)]);
+        return {{p2(d.x, d.x), p2(d.y, d.y), p2(-d.x, -d.x), p2(-d.y, -d.y)}};
+    }
+};
+
+// Per-CTA sums of a pass: warp shuffles, then one value per warp.
+template <bool FIRST>
+__device__ __forceinline__ void zzx_sums(double e, double q, double* __restrict__ partial) {
+    const unsigned t = threadIdx.x;
 #pragma unroll
     for (int w = 16; w > 0; w >>= 1) {
         e += __shfl_down_sync(0xffffffffu, e, w);
@@ -257,6 +220,181 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
         for (int w = 0; w < ZZX_THREADS / 32; ++w) s += sums[t][w];
         partial[t * gridDim.x + blockIdx.x] = s;
     }
+}
+
+// H psi and the energy. FIRST: the diagonal and the 11 lowest bits; otherwise the bits of p.terms
+// (above the 3 lowest). psi's copy goes to phi and H psi to lam, both in the sweep's layout
+// (P::put); later passes read phi and add to lam. Without VEC only the energy is formed (complex64;
+// the next tile's amplitudes are loaded while this one is worked on: 14.7 -> 12.6 ms at 30 qubits,
+// with a pass that takes all its bits not testing each; and complex128 below 22 qubits). partial[blockIdx] gets the
+// pass's share of Re <psi|H psi>, and with FIRST partial[gridDim + blockIdx] that of <psi|psi>.
+template <class P, bool FIRST, bool VEC>
+__global__ void __launch_bounds__(ZZX_THREADS, sizeof(typename P::S) == 8 ? (VEC ? 4 : 2) : FIRST ? 2 : 3)
+k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
+      typename P::S* __restrict__ lam, const __grid_constant__ ZzxParams p,
+      double* __restrict__ partial) {
+    using V = typename P::V;
+    __shared__ __align__(16) V tile[1 << ZZX_BITS];
+    __shared__ ZzxDiag diag;
+    const unsigned t = threadIdx.x;
+    if (FIRST) diag.tables(p, t);
+    bool large = false;
+    PDot2 acc, nrm;
+    acc.s = acc.en = nrm.s = nrm.en = 0;
+    typename P::S raw[ZZX_REGS];
+    auto load = [&](uint64_t g) {
+        uint64_t base, step;
+        zzx_place<FIRST>(p, g, t, base, step);
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) raw[j] = psi[base + j * step];
+    };
+    if (!VEC && blockIdx.x < p.ntiles) load(blockIdx.x);
+    for (uint64_t g = blockIdx.x; g < p.ntiles; g += gridDim.x) {
+        uint64_t base, step;
+        zzx_place<FIRST>(p, g, t, base, step);
+        V v[ZZX_REGS];
+        if constexpr (!FIRST && VEC) {
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) v[j] = P::get(phi + base + j * step);
+        } else {
+            if (VEC) load(g);
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) {
+                v[j] = P::split(raw[j]);
+                if constexpr (FIRST) large = large || P::too_large(raw[j]);
+            }
+        }
+        __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) tile[t + ZZX_THREADS * j] = v[j];
+        if (!VEC && g + gridDim.x < p.ntiles) load(g + gridDim.x);
+        if (FIRST) diag.above(p, g, t);
+        __syncthreads();
+        // (a pass that takes all bits of its tile, as all but the last do, tests none of them)
+        auto work = [&](auto every) {
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) {
+                typename P::Sum s;
+                if constexpr (FIRST) {
+                    s.first(diag.entry(t, j).c, v[j]);
+                } else {
+                    const u64 zero[4] = {0, 0, 0, 0};
+                    s.first(zero, v[j]);
+                }
+#pragma unroll
+                for (int m = FIRST ? 0 : ZZX_LOW; m < 8; ++m)
+                    if (decltype(every)::value || ((p.terms >> m) & 1u))
+                        s.add(p.x[m].c, tile[(t ^ (1u << m)) + ZZX_THREADS * j]);
+#pragma unroll
+                for (int m = 8; m < ZZX_BITS; ++m)
+                    if (decltype(every)::value || ((p.terms >> m) & 1u)) s.add(p.x[m].c, v[j ^ (1 << (m - 8))]);
+                const V o = s.result();
+                P::term(acc, v[j], o);
+                if constexpr (FIRST) P::term(nrm, v[j], v[j]);
+                if constexpr (VEC) {
+                    if constexpr (FIRST) {
+                        P::put(phi + base + j * step, v[j]);
+                        P::put(lam + base + j * step, o);
+                    } else {
+                        P::put(lam + base + j * step, P::plus(P::get(lam + base + j * step), o));
+                    }
+                }
+            }
+        };
+        if constexpr (FIRST) {
+            work(std::true_type{});
+        } else {
+            if (p.terms == (1u << ZZX_BITS) - (1u << ZZX_LOW)) work(std::true_type{});
+            else work(std::false_type{});
+        }
+    }
+    zzx_sums<FIRST>(zzx_value(acc), FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0, partial);
+}
+
+// The energy alone, complex128: the X term of bit m is 2 c_m sum Re conj(psi[x]) psi[x ^ 2^m] over the pairs,
+// one product per pair where H psi takes two per amplitude (half the operations), summed per bit
+// and weighted once per thread in f64. Three bits at a time lie in a thread's registers: the tile
+// is written to shared memory once and read in three more arrangements (two in a later pass), 24
+// reads of an amplitude per thread instead of one per bit. Energy call: 24 qubits 520 -> 382 us, 30
+// qubits 38.0 -> 26.1 ms (8.9 of them the reads at HBM speed; L2 prefetches of the next tile cost 4).
+// Not for complex64, whose H psi takes one operation per amplitude and bit (18.1 against 12.6 ms).
+template <bool FIRST>
+__global__ void __launch_bounds__(ZZX_THREADS, 2)
+k_zzx_energy(const double2* __restrict__ psi, const __grid_constant__ ZzxParams p,
+             double* __restrict__ partial) {
+    using P = ZvFF;
+    using V = typename P::V;
+    __shared__ __align__(16) V tile[1 << ZZX_BITS];
+    __shared__ ZzxDiag diag;
+    const unsigned t = threadIdx.x;
+    if (FIRST) diag.tables(p, t);
+    bool large = false;
+    PDot2 acc, nrm, bit[ZZX_BITS];
+    acc.s = acc.en = nrm.s = nrm.en = 0;
+#pragma unroll
+    for (int m = 0; m < ZZX_BITS; ++m) bit[m].s = bit[m].en = 0;
+    const unsigned at0 = P::place(t), at1 = P::place((t & 31u) | ((t >> 5) << 8)),
+                   at2 = P::place((t & 3u) | ((t >> 2) << 5)), at3 = P::place(t << 3);
+    for (uint64_t g = blockIdx.x; g < p.ntiles; g += gridDim.x) {
+        uint64_t base, step;
+        zzx_place<FIRST>(p, g, t, base, step);
+        V v[ZZX_REGS];
+        typename P::S raw[ZZX_REGS];
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) raw[j] = psi[base + j * step];
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) {
+            v[j] = P::split(raw[j]);
+            if constexpr (FIRST) large = large || P::too_large(raw[j]);
+        }
+        __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) tile[at0 ^ P::place(ZZX_THREADS * j)] = v[j];
+        if (FIRST) diag.above(p, g, t);
+        __syncthreads();
+        if constexpr (FIRST) {
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) {
+                typename P::Sum s;
+                s.first(diag.entry(t, j).c, v[j]);
+                P::term(acc, v[j], s.result());
+                P::term(nrm, v[j], v[j]);
+            }
+        }
+        // the pairs of tile bits m0 .. m0 + 2, in register bits 0 .. 2
+        auto pairs = [&](auto m0) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                constexpr int M0 = decltype(m0)::value;
+                if (!((p.terms >> (M0 + k)) & 1u)) continue;
+#pragma unroll
+                for (int j = 0; j < ZZX_REGS; ++j)
+                    if (!(j & (1 << k))) P::term(bit[M0 + k], v[j], v[j | (1 << k)]);
+            }
+        };
+        pairs(std::integral_constant<int, 8>{});
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at1 ^ P::place(j << 5)];
+        pairs(std::integral_constant<int, 5>{});
+#pragma unroll
+        for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at2 ^ P::place(j << 2)];
+        pairs(std::integral_constant<int, 2>{});
+        if constexpr (FIRST) {
+#pragma unroll
+            for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at3 ^ P::place(j)];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (!((p.terms >> k) & 1u)) continue;
+#pragma unroll
+                for (int j = 0; j < ZZX_REGS; ++j)
+                    if (!(j & (1 << k))) P::term(bit[k], v[j], v[j | (1 << k)]);
+            }
+        }
+    }
+    double e = FIRST ? zzx_value(acc) : 0.0;
+#pragma unroll
+    for (int m = FIRST ? 0 : ZZX_LOW; m < ZZX_BITS; ++m) e = fma(p.twice[m], zzx_value(bit[m]), e);
+    zzx_sums<FIRST>(e, FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0, partial);
 }
 
 // out[r] = sum of row r (nb values each): one warp per row, fixed order
@@ -286,9 +424,12 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
     static_assert(1 + (MAX_HAM_QUBITS - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD + 1 <= 8, "row sums");
     const int npass = 1 + (n - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD;
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx<P, true, VEC>, ZZX_THREADS, 0) !=
-            cudaSuccess || occ < 1)
-        occ = 1;
+    bool pairs = false;  // k_zzx_energy
+    if constexpr (!VEC && sizeof(typename P::S) == 16) pairs = n >= ZZX_PAIRS_QUBITS;
+    cudaError_t e;
+    if (pairs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx_energy<true>, ZZX_THREADS, 0);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx<P, true, VEC>, ZZX_THREADS, 0);
+    if (e != cudaSuccess || occ < 1) occ = 1;
     const uint64_t ntiles = h->dim >> ZZX_BITS;
     const int nb = (int)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * occ);
     int st = h->work.ensure(((size_t)(npass + 1) * nb + npass + 1) * sizeof(double));
@@ -310,10 +451,12 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
             p.shift = first;
         }
         p.terms = 0;
+        std::memset(p.twice, 0, sizeof(p.twice));
         for (int m = low; m < ZZX_BITS; ++m) {
             const int bit = first + m - low;
             if (bit < done || bit >= n) continue;
             p.terms |= 1u << m;
+            p.twice[m] = 2.0 * H.b[n - 1 - bit];
             const float2 c = coef_pair(H.b[n - 1 - bit]);
             p.x[m].c[0] = both(c.x);
             p.x[m].c[1] = both(c.y);
@@ -321,11 +464,16 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
             p.x[m].c[3] = both(-c.y);
         }
         done = first + ZZX_BITS - low;
-        if (pass == 0)
-            k_zzx<P, true, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, partial);
-        else
-            k_zzx<P, false, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(
-                psi, phi, lam, p, partial + (size_t)(pass + 1) * nb);
+        double* row = partial + (pass == 0 ? 0 : (size_t)(pass + 1) * nb);
+        if (pairs) {
+            if constexpr (sizeof(typename P::S) == 16) {
+                if (pass == 0) k_zzx_energy<true><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
+                else k_zzx_energy<false><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
+            }
+        } else {
+            if (pass == 0) k_zzx<P, true, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, row);
+            else k_zzx<P, false, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, row);
+        }
         QGPU_CHECK_LAUNCH("k_zzx");
         h->launches++;
         h->h2d_bytes += sizeof(p);
