@@ -11,7 +11,7 @@
 //      i.i.d. Exp(1) and S_k their prefix sums, (S_0, ..., S_{N-1}) / S_N is distributed as the
 //      order statistics of N i.i.d. U(0, 1); Devroye, "Non-Uniform Random Variate Generation",
 //      1986, V.2), so the sampled indices come out sorted and the histogram is a run-length pass.
-//   4. k_sample: one warp per shot: binary search over chunk offsets, then the same lane/warp
+//   4. k_sample: one lane per shot: binary search over chunk offsets, then the same lane/warp
 //      cumulative sums as step 1 locate the first index whose cumulative probability exceeds u.
 // All sums are f64.
 #include <algorithm>
@@ -46,25 +46,46 @@ __device__ __forceinline__ double warp_incl_scan(double v) {
     return v;
 }
 
-// Lane sum of the lane's run of a chunk (sequential, like the reference's running sum).
+// The probabilities of a chunk into a warp's part of shared memory, loaded in runs of a warp's width
+// (each lane reading its own run of 16 amplitudes touches 32 lines per load), one pad per 16 so that
+// the lanes' runs lie in different banks.
+constexpr int CHUNK_PAD = (1 << CHUNK_BITS) + (1 << CHUNK_BITS) / 16;
+constexpr int MEASURE_WARPS = 8;  // per CTA
+__device__ __forceinline__ int chunk_at(int q) { return q + (q >> 4); }
 template <class S>
-__device__ __forceinline__ double lane_run_sum(const S* st, uint64_t first, int count) {
+__device__ __forceinline__ void load_chunk(const S* st, uint64_t first, int chunk_len, double* p) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();  // readers of the chunk before are done
+    if (chunk_len == 1 << CHUNK_BITS) {
+#pragma unroll
+        for (int q = 0; q < 1 << CHUNK_BITS; q += 32) p[chunk_at(q + lane)] = prob(st, first + q + lane);
+    } else {
+        for (int q = lane; q < chunk_len; q += 32) p[chunk_at(q)] = prob(st, first + q);
+    }
+    __syncwarp();
+}
+
+// Lane sum of the lane's run of a loaded chunk (sequential, like the reference's running sum).
+__device__ __forceinline__ double lane_run_sum(const double* p, int per_lane, int chunk_len) {
+    const int first = (threadIdx.x & 31) * per_lane;
     double s = 0.0;
-    for (int q = 0; q < count; ++q) s = __dadd_rn(s, prob(st, first + q));
+    if (first < chunk_len)
+        for (int q = 0; q < per_lane; ++q) s = __dadd_rn(s, p[chunk_at(first + q)]);
     return s;
 }
 
 template <class S>
 __global__ void k_chunk_sums(const S* __restrict__ st, uint64_t nchunks, int chunk_len,
                              double* __restrict__ sums) {
+    __shared__ double chunk[MEASURE_WARPS][CHUNK_PAD];
+    double* p = chunk[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const int per_lane = chunk_len >> 5 ? chunk_len >> 5 : 1;
     for (uint64_t c = warp; c < nchunks; c += nwarps) {
-        const uint64_t first = c * (uint64_t)chunk_len + (uint64_t)lane * per_lane;
-        const double s = (lane * per_lane < chunk_len) ? lane_run_sum(st, first, per_lane) : 0.0;
-        const double inc = warp_incl_scan(s);
+        load_chunk(st, c * (uint64_t)chunk_len, chunk_len, p);
+        const double inc = warp_incl_scan(lane_run_sum(p, per_lane, chunk_len));
         if (lane == 31) sums[c] = inc;
     }
 }
@@ -147,62 +168,73 @@ __global__ void k_normalise(const double* __restrict__ ex_scan, const double* __
     u[i] = __ddiv_rn(__dadd_rn(ex_scan[i], e[i]), *total);
 }
 
+// A warp takes `per_warp` (1 .. 32) consecutive shots, each lane the binary search, the scan over the
+// chunk's lane ends and the walk of one of them; a chunk that several of them hit is loaded once.
+// Bound: latency of the searches. The whole call, against a warp per shot (all lanes in one search,
+// a chunk read per shot in uncoalesced runs): 18 qubits, 20000 shots 300 -> 175 us; 24 qubits, 10^6
+// shots 11.0 -> 2.2 ms; unchanged where each shot hits a chunk of its own (24 qubits, 1000 shots
+// 0.25 ms, 30 qubits, 256 shots 9.0 ms: the FP64 operations of k_chunk_sums).
 template <class S>
-__global__ void k_sample(const S* __restrict__ st, uint64_t dim, const double* __restrict__ offs,
+__global__ void k_sample(const S* __restrict__ st, const double* __restrict__ offs,
                          const double* __restrict__ sums, uint64_t nchunks, int chunk_len,
-                         const double* __restrict__ u, uint64_t nshots, int64_t* __restrict__ out) {
+                         const double* __restrict__ u, uint64_t nshots, int per_warp,
+                         int64_t* __restrict__ out) {
+    __shared__ double chunk[MEASURE_WARPS][CHUNK_PAD];
+    __shared__ double scans[MEASURE_WARPS][32];
+    double* p = chunk[threadIdx.x >> 5];
+    double* inc = scans[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const int per_lane = chunk_len >> 5 ? chunk_len >> 5 : 1;
-    for (uint64_t s = warp; s < nshots; s += nwarps) {
-        const double x = u[s];
+    const int lanes = chunk_len < 32 ? chunk_len : 32;  // lanes that hold amplitudes of a chunk
+    for (uint64_t s0 = warp * per_warp; s0 < nshots; s0 += nwarps * per_warp) {
+        const uint64_t s = s0 + lane;
+        const bool mine = lane < per_warp && s < nshots;
+        const double x = mine ? u[s] : 0.0;
         // first chunk c with x < offs[c] + sums[c]
-        uint64_t lo = 0, hi = nchunks;
+        uint64_t lo = 0, hi = mine ? nchunks : 0;
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
             if (x < __dadd_rn(offs[mid], sums[mid])) hi = mid;
             else lo = mid + 1;
         }
-        if (lo == nchunks) {
-            if (lane == 0) out[s] = -1;  // `measure` returns None: u reached the total
-            continue;
-        }
-        const uint64_t c = lo;
-        const uint64_t first = c * (uint64_t)chunk_len + (uint64_t)lane * per_lane;
-        const bool active = lane * per_lane < chunk_len;
-        const double ls = active ? lane_run_sum(st, first, per_lane) : 0.0;
-        const double inc = warp_incl_scan(ls);
-        const double start = __dadd_rn(offs[c], inc - ls);  // lane's exclusive offset
-        const double excl = __shfl_up_sync(0xffffffffu, inc, 1);
-        const double lane_start = __dadd_rn(offs[c], lane == 0 ? 0.0 : excl);
-        (void)start;
-        const double lane_end = __dadd_rn(offs[c], inc);
-        const unsigned hit = __ballot_sync(0xffffffffu, active && x < lane_end);
-        int64_t result;
-        if (hit) {
-            const int L = __ffs(hit) - 1;
-            // lane L walks its run sequentially
-            int64_t idx = -1;
-            if (lane == L) {
-                double cum = lane_start;
-                const uint64_t f = c * (uint64_t)chunk_len + (uint64_t)L * per_lane;
-                int64_t last_nz = (int64_t)f + per_lane - 1;
-                for (int q = 0; q < per_lane; ++q) {
-                    const double p = prob(st, f + q);
-                    cum = __dadd_rn(cum, p);
-                    if (x < cum) { idx = (int64_t)(f + q); break; }
-                    if (p > 0.0) last_nz = (int64_t)(f + q);
+        if (mine && lo == nchunks) out[s] = -1;  // `measure` returns None: u reached the total
+        unsigned left = __ballot_sync(0xffffffffu, mine && lo < nchunks);
+        while (left) {
+            const uint64_t c = __shfl_sync(0xffffffffu, lo, __ffs(left) - 1);
+            load_chunk(st, c * (uint64_t)chunk_len, chunk_len, p);
+            inc[lane] = warp_incl_scan(lane_run_sum(p, per_lane, chunk_len));
+            __syncwarp();
+            const bool here = ((left >> lane) & 1u) && lo == c;
+            if (here) {
+                const double off = offs[c];
+                int L = 0;  // first lane whose run ends above x
+                while (L < lanes && !(x < __dadd_rn(off, inc[L]))) ++L;
+                int64_t idx = -1;
+                if (L < lanes) {
+                    double cum = __dadd_rn(off, L == 0 ? 0.0 : inc[L - 1]);
+                    const int64_t f = (int64_t)(c * (uint64_t)chunk_len) + L * per_lane;
+                    int64_t last_nz = f + per_lane - 1;
+                    for (int q = 0; q < per_lane; ++q) {
+                        const double v = p[chunk_at(L * per_lane + q)];
+                        cum = __dadd_rn(cum, v);
+                        if (x < cum) {
+                            idx = f + q;
+                            break;
+                        }
+                        if (v > 0.0) last_nz = f + q;
+                    }
+                    if (idx < 0) idx = last_nz;  // rounding edge between the two sum orders
+                } else {
+                    // x lies below the chunk's end by the chunk-sum ordering but above every lane
+                    // end by the lane ordering (last-bit disagreement): take the chunk's last index.
+                    idx = (int64_t)((c + 1) * (uint64_t)chunk_len - 1);
                 }
-                if (idx < 0) idx = last_nz;  // rounding edge between the two sum orders
+                out[s] = idx;
             }
-            result = __shfl_sync(0xffffffffu, idx, L);
-        } else {
-            // x lies below the chunk's end by the chunk-sum ordering but above every lane end
-            // by the lane ordering (last-bit disagreement): take the chunk's last index.
-            result = (int64_t)((c + 1) * (uint64_t)chunk_len - 1);
+            left &= ~__ballot_sync(0xffffffffu, here);
         }
-        if (lane == 0) out[s] = result;
     }
 }
 
@@ -247,16 +279,19 @@ static int build_cdf(qgpu_handle* h, size_t extra_doubles, Cdf* c) {
 }
 
 static int run_sample(qgpu_handle* h, const Cdf& c, const double* u, uint64_t n, int64_t* out) {
-    const int threads = 256;
-    uint64_t blocks = (n * 32 + threads - 1) / threads;
+    const int threads = 32 * MEASURE_WARPS;
+    // one shot per warp until 16 warps per SM are busy, then as many as that takes (up to 32)
+    const uint64_t warps = (uint64_t)h->sm_count * 16;
+    const int per_warp = (int)std::min<uint64_t>(32, std::max<uint64_t>(1, n / warps));
+    uint64_t blocks = ((n + per_warp - 1) / per_warp * 32 + threads - 1) / threads;
     if (blocks > (uint64_t)h->sm_count * 32) blocks = (uint64_t)h->sm_count * 32;
     if (blocks < 1) blocks = 1;
     if (h->precision == QGPU_C128)
         k_sample<double2><<<(unsigned)blocks, threads, 0, h->stream>>>(
-            (const double2*)h->state, h->dim, c.offs, c.sums, c.nchunks, c.chunk_len, u, n, out);
+            (const double2*)h->state, c.offs, c.sums, c.nchunks, c.chunk_len, u, n, per_warp, out);
     else
         k_sample<float2><<<(unsigned)blocks, threads, 0, h->stream>>>(
-            (const float2*)h->state, h->dim, c.offs, c.sums, c.nchunks, c.chunk_len, u, n, out);
+            (const float2*)h->state, c.offs, c.sums, c.nchunks, c.chunk_len, u, n, per_warp, out);
     QGPU_CHECK_LAUNCH("k_sample");
     h->launches++;
     return QGPU_OK;
