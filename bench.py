@@ -546,16 +546,16 @@ def mode_summary(prof, ms, steps, gbytes, peak) -> dict:
 
 def reference_precision_leg(args, nat, prog, fast_handle, gbytes, peak, dev) -> dict:
     """The same circuit in QGPU_MODE_F64 (native f64 FMA, the fast mode's plan) and in
-    QGPU_MODE_EXACT (one pass per gate, f64 products and sums in the reference's order: equal to
-    the oracle value for value), each timed, then compared on the device with the fast-mode
+    QGPU_MODE_EXACT (f64 products and sums in the reference's order: equal to the oracle value for
+    value), each timed, then compared on the device with the fast-mode
     result: max |a_fast - a_exact|, max |a_f64 - a_exact|, 1 - fidelity and norm drift, without
     downloading the 16 GiB registers."""
     out = {}
     hx, ms_x, prof_x = timed_simulation(nat, args.n, prog, nat.QGPU_C128, nat.QGPU_MODE_EXACT,
                                         0, 1, dev)
-    if not prof_x:  # exact mode: one k_group pass per non-identity gate over the whole register
-        ng = int((prog.ops["kind"] != 0).sum())
-        prof_x = {"k_group": [ng, ms_x, ng * 32.0 * (1 << args.n)]}
+    if not prof_x:  # exact mode: k_exact passes over the whole register, beside two set_zero launches
+        passes = hx.launch_count() - 2
+        prof_x = {"k_exact": [passes, ms_x, passes * 32.0 * (1 << args.n)]}
     out["exact"] = mode_summary(prof_x, ms_x, 1, gbytes, peak)
     out["exact"].update({"steps": 1, "warmup": 0, "norm_drift": hx.norm() - 1.0})
     hf, ms_f, prof_f = timed_simulation(nat, args.n, prog, nat.QGPU_C128, nat.QGPU_MODE_F64,

@@ -2,15 +2,17 @@
 // (src/circuit/simulation.rs:21-57) and `apply_gate` (simulation.rs:64-135).
 //
 // Two execution paths:
-//  * QGPU_MODE_EXACT (complex128): one launch of k_group per gate. Each CTA stages whole
-//    gate groups (the 2^k amplitudes that share all non-acting bits) in shared memory and writes
-//    out[l] = none[l] ? a[l] : sum over non-None inputs j, in increasing full index, of
-//    M[l][j] * a[j] — f64 products and sums without contraction, first product assigned then
-//    added to (simulation.rs:168-179) — so amplitudes equal the reference's.
+//  * QGPU_MODE_EXACT (complex128): runs of standard gates in tile passes (exact.cu); from the first
+//    Custom gate on, one launch of k_group per gate. Each CTA stages whole gate groups (the 2^k
+//    amplitudes that share all non-acting bits) in shared memory and writes out[l] =
+//    none[l] ? a[l] : sum over non-None inputs j, in increasing full index, of M[l][j] * a[j] —
+//    f64 products and sums without contraction, first product assigned then added to
+//    (simulation.rs:168-179) — so amplitudes equal the reference's.
 //  * fused (QGPU_MODE_FAST / QGPU_MODE_F64 / complex64): the planner (plan.cpp) turns the gate
-//    list into register-tile passes. k_tile<K> gives each thread 2^K amplitudes that differ in
-//    the pass's K tile bits, applies every step of the pass in registers and writes them back:
-//    one HBM round trip per pass.
+//    list into passes. Wide passes (wide.cuh) hold a tile in shared memory and take many gates;
+//    pair blocks of large registers run in digits (digits.cu); k_tile<K> gives each thread 2^K
+//    amplitudes that differ in the pass's K tile bits, applies every step of the pass in registers
+//    and writes them back: one HBM round trip per pass.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
