@@ -203,6 +203,7 @@ struct AGate {
     int a = 0, b = 0;   // SWAP bits; PAIR: hi, lo bits
     int block = -1;     // BLOCK: index into plan.customs; PAIR: index into plan.pairs
     uint64_t support = 0;  // all bits the gate reads or writes
+    bool given = false;    // u holds entries of a Custom gate (PAIR: see its block)
 };
 
 int unit_code(cd x) {
@@ -409,6 +410,7 @@ std::vector<AGate> fuse_pairs(const std::vector<AGate>& gates, int n, Plan* plan
         for (int r = 0; r < 4; ++r)
             for (int c = 0; c < 4; ++c) acc[r][c] = r == c ? 1.0 : 0.0;
         for (int gi : o.members) {  // acc <- G * acc, in circuit order
+            pb.given = pb.given || gates[gi].given;
             cd gm[4][4], nx[4][4];
             pair_matrix(gates[gi], pb.hi, pb.lo, gm);
             for (int r = 0; r < 4; ++r)
@@ -563,6 +565,7 @@ void emit_one(const AGate& g, std::vector<HStep>& out) {
             h.d0 = u00;
             h.d1 = u11;
         }
+        h.s.given = g.given;
         out.push_back(h);
         return;
     }
@@ -578,6 +581,7 @@ void emit_one(const AGate& g, std::vector<HStep>& out) {
     } else {
         h.s = blank_step(ST_DENSE);
     }
+    h.s.given = g.given;
     h.s.cm = g.cm;
     set_entry(h.s, 0, u00);
     set_entry(h.s, 1, u01);
@@ -1294,6 +1298,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
                 for (int in = 0; in < 2; ++in)
                     r[lo][in] = a.u[lo][0] * p.u[0][in] + a.u[lo][1] * p.u[1][in];
             std::memcpy(p.u, r, sizeof(r));
+            p.given = p.given || a.given;
             return;
         }
         close_bits(a.support);
@@ -1369,6 +1374,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
         }
         AGate a;
         a.kind = AGate::ONE;
+        a.given = op.kind == QGPU_GATE_CUSTOM;
         a.t = bitpos[k - 1];
         a.cm = support & ~(1ull << a.t);
         a.support = support;

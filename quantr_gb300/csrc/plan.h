@@ -112,7 +112,9 @@ struct DevStep {
     uint64_t cm;                       // control mask on the full index
     uint32_t tab_off[MAX_TABLE_FIELDS];  // TABLE: entry offsets into the pass table buffer
     uint8_t tab_shift[MAX_TABLE_FIELDS], tab_width[MAX_TABLE_FIELDS];
-    uint8_t nfields, pad[3];
+    uint8_t nfields;
+    uint8_t given;                     // entries (or a factor of them) come from a Custom gate
+    uint8_t pad[2];
     float ff[16];                      // up to 4 complex entries as float pairs
     double d[8];                       // the same entries in f64
     // Packed f32x2 operands of the float-pair kernels: term t of a Dot2 uses
@@ -170,6 +172,7 @@ struct Pass {
 // (terms (Re, Re) on x_c and (-Im, Im) on swap(x_c), 4 slots each as in DevStep::pk).
 struct PairBlock {
     int hi = 0, lo = 0;
+    bool given = false;                // a Custom gate is among its factors
     cd m[4][4];                        // m[out][in]
     uint64_t pk[128];
 };

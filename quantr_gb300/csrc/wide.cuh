@@ -423,6 +423,9 @@ static u64 wide_pack(float x, float y) {
 // A step's constants. Rounding an unconditional 2x2 or 4x4 changes the register's norm a little
 // (f64 rounding already does: 1e-14 over 200 rotations): *drift is the relative change so far, and
 // the next such step takes it out before it is rounded, so that it does not grow with the gates.
+// A step of library gates is unitary but for its rounding; what a Custom gate's entries are off a
+// unitary matrix belongs to the gate, so there only the entries' split into floats counts (240 gates
+// scaling by 1 - 6.7e-14 each otherwise came out as if they did not).
 template <class A>
 static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, double* drift) {
     constexpr bool ff = sizeof(typename A::V) == 16;
@@ -449,16 +452,26 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
     const bool pair32 = !ff && s.type == ST_DENSE4;  // (complex64 pair blocks: hi alone)
     const bool whole = s.cm == 0 && (s.type == ST_REAL || s.type == ST_DENSE || s.type == ST_DENSE4);
     const bool third_kept = ff && s.type != ST_DENSE && s.type != ST_DENSE4;
-    double size = 0.0, off = 0.0, exact = 0.0;  // sums of x^2, of x (x' - x), and of x^2's rounding
+    const bool given = s.given || (s.type == ST_DENSE4 && plan.pairs[ws.pair].given);
+    double size = 0.0, exact = 0.0;  // sum of x^2 over the entries, and its rounding
+    for (cd z : e)
+        for (double x : {z.real(), z.imag()}) {
+            const double sq = x * x, sum = size + sq, b = sum - size;
+            exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
+            size = sum;
+        }
+    // sum |e|^2 of a unitary d x d matrix is d (false for sizes that are not finite)
+    const double d = given ? size : s.type == ST_DENSE4 ? 4.0 : s.type == ST_PHASE ? 1.0 : 2.0;
+    const bool known = given ? size > 0.0 && size < HUGE_VAL : std::fabs(size - d) < 1e-12;
+    const double off = given ? 0.0 : (size - d) + exact;
+    double change = 0.0;  // sum of x'^2 - x^2 for the entries x' that are uploaded
     auto part = [&](double x, float* h, float* l, float* third) {
-        *h = (float)x;
-        *l = pair32 ? 0.0f : (float)(x - (double)*h);
-        *third = (float)((x - (double)*h) - (double)*l);
+        const double y = whole && known ? x - x * *drift : x;
+        *h = (float)y;
+        *l = pair32 ? 0.0f : (float)(y - (double)*h);
+        *third = (float)((y - (double)*h) - (double)*l);
         const double kept = ((double)*h + (double)*l) + (third_kept ? (double)*third : 0.0);
-        const double sq = x * x, sum = size + sq, b = sum - size;
-        exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
-        size = sum;
-        off += x * (kept - x);
+        change += (kept - x) * (kept + x);
     };
     auto term = [&](float h, float l, float third, bool mixed) {  // hi, -third, -hi, -lo
         const float s0 = mixed ? -1.0f : 1.0f;  // (the real lane of an imaginary part)
@@ -468,7 +481,6 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
         c.push_back(wide_pack(-s0 * l, -l));
     };
     for (cd z : e) {
-        if (whole) z -= z * *drift;
         float rh, rl, r3, ih, il, i3;
         part(z.real(), &rh, &rl, &r3);
         part(z.imag(), &ih, &il, &i3);
@@ -482,11 +494,9 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
             if (s.type != ST_REAL && !pair32) c.push_back(wide_pack(il, il));
         }
     }
-    // sum |e|^2 of a unitary d x d matrix is d: half the relative error of it, and the rounding's
-    const double d = s.type == ST_DENSE4 ? 4.0 : 2.0;
-    if (whole && std::fabs(size - d) < 1e-12) *drift += 0.5 * ((size - d) + exact) / d + off / d;
-    if (s.type == ST_PHASE && __builtin_popcountll(s.cm) == 1 && std::fabs(size - 1.0) < 1e-12)
-        *drift += 0.25 * ((size - 1.0) + exact) + 0.5 * off;  // (half the amplitudes)
+    if (whole && known) *drift += 0.5 * (off + change) / d;
+    if (s.type == ST_PHASE && !s.unit && known && __builtin_popcountll(s.cm) == 1)
+        *drift += 0.25 * (off + change) / d;  // (half the amplitudes)
     if (c.size() & 1) c.push_back(0);  // 16-byte aligned
     return c;
 }

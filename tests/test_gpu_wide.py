@@ -8,6 +8,7 @@ import pytest
 
 from quantr_gb300 import _native as nat
 from quantr_gb300 import workloads as W
+from quantr_gb300.program import ProgramBuilder
 from test_wide_host import _everything
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,37 @@ def _small(n):
         b.add("CNot", 0, (1,))
         b.add("Ry", 0, (), param=2.5)
     return b.build()
+
+
+def _chain(kind, n, layers):
+    """Custom gates that are nearly, but not exactly, unitary, in every layer."""
+    r = np.random.default_rng(11)
+    b = ProgramBuilder(n)
+    none = np.zeros(2, np.uint8)
+    c, s = np.cos(0.4), np.sin(0.4)
+    matrix = {"real": np.full((2, 2), 0.7071067811865) * [[1, 1], [1, -1]],  # 13 digits of sqrt(1/2)
+              "complex": (1.0 - 1.6e-13) * np.array([[c, -s], [1j * s, 1j * c]]),
+              "phase": np.diag([1.0, 1.0 - 4e-13])}  # damps |1>
+    matrix["grown"] = matrix["real"]
+    for w in range(n):
+        b.add("Ry", w, (), param=r.uniform(0.3, 2.8))
+    for layer in range(layers):
+        for w in range(n):
+            b.add_custom(w, [], matrix[kind].astype(np.complex128), none)
+            if kind == "grown" and layer == layers // 2:  # not unitary at all, in between
+                b.add_custom(w, [], np.array([[1.25, 0.25], [-0.5, 0.75]], np.complex128), none)
+            if kind == "phase":  # (Toffoli gates keep the steps apart)
+                b.add("Toffoli", w, ((w + 3) % n, (w + 7) % n))
+                b.add("Ry", w, (), param=r.uniform(-0.2, 0.2))
+                b.add("Toffoli", w, ((w + 2) % n, (w + 5) % n))
+        for w in range(n):
+            b.add("CNot", (w + 1) % n, (w,))
+    return b.build()
+
+
+@pytest.mark.parametrize("kind", ["real", "complex", "phase", "grown"])
+def test_custom_gates_keep_their_scaling(oracle, kind):
+    """What a Custom matrix is off a unitary one belongs to the gate: 240 of them scale amplitudes by 1 -
+    1.6e-11 and more, which is not taken for the rounding of library gates."""
+    prof = _check(oracle, _chain(kind, 12, 20), nat.QGPU_C128)
+    assert any(k.startswith("k_wide") for k in prof), prof
