@@ -123,17 +123,22 @@ __global__ void __launch_bounds__(1024) k_exact(double2* __restrict__ st, const 
     }
 }
 
-// One gate with full-index bits; false for forms no standard gate takes.
+// One gate with full-index bits.
 struct ExGate {
     ExOp op;
     int bit = 0, bit2 = -1;
     uint64_t cm = 0, need = 0;
 };
 
+// False for forms no standard gate takes and for entries that are not finite: of an angle's NaN or
+// infinity some amplitudes become NaN, and the products with 0 of this gate and the next ones spread
+// them.
 static bool exact_gate(const qgpu_op& op, const LocalGate& lg, int n, ExGate* g) {
     std::memset(&g->op, 0, sizeof(g->op));
     const int k = lg.k;
     const size_t d = (size_t)1 << k, call = (d - 1) & ~(size_t)1;
+    for (cd z : lg.M)
+        if (!std::isfinite(z.real()) || !std::isfinite(z.imag())) return false;
     g->bit = n - 1 - lg.wires[k - 1];
     if (op.kind == QGPU_GATE_SWAP) {
         g->op.type = EX_SWAP;

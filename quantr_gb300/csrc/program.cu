@@ -2124,8 +2124,8 @@ extern "C" int qgpu_apply_program(qgpu_handle* h, const qgpu_op* ops, size_t n_o
             at.push_back(g);
         }
         // Tile passes leave out products with 0 and 1, which on finite amplitudes changes no value:
-        // they take the gates up to the first Custom one when the register's norm is known or found
-        // to be finite and far from overflow. The rest goes through one launch per gate.
+        // they take the gates up to the first Custom one (or one whose entries are not finite) when the
+        // register's norm is known or found to be finite and far from overflow. The rest goes through one launch per gate.
         size_t taken = 0;
         if (!gates.empty() && ops[at[0]].kind != QGPU_GATE_CUSTOM) {
             double bound = bound_before;

@@ -94,3 +94,24 @@ def test_registers_that_are_not_finite(oracle):
     out, launches = _run(prog, reg)
     assert launches >= len(prog.ops)
     assert np.array_equal(out, oracle.simulate(prog, reg, engine=oracle.DENSE), equal_nan=True)
+
+
+@pytest.mark.parametrize("angle", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("kind", ["CR", "Rz", "Ry"])
+def test_angles_that_are_not_finite(oracle, kind, angle):
+    """A NaN that a gate's entry brings in spreads through the products with 0 of the gates after it
+    (H, H, CR(NaN), CNot: all four amplitudes)."""
+    b = ProgramBuilder(3)
+    for w in range(3):
+        b.add("H", w)
+    if kind == "CR":
+        b.add("CR", 1, (0,), param=angle)
+    else:
+        b.add(kind, 1, (), param=angle)
+    b.add("CNot", 2, (1,))
+    b.add("T", 0)
+    prog = b.build()
+    out, _ = _run(prog)
+    ref = oracle.simulate(prog, engine=oracle.DENSE)
+    assert np.isnan(ref).any()
+    assert np.array_equal(out, ref, equal_nan=True)
