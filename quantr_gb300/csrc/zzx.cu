@@ -50,17 +50,17 @@ struct ZzxParams {
     // the diagonal (first pass): ZZ coefficient of bits (q, q+1) and of the wrap (0, n-1)
     float2 zz[MAX_HAM_QUBITS];
     float2 wrap;
-    double twice[ZZX_BITS];     // twice the X coefficient of tile bit m (0: not this pass's)
+    u64 twice[ZZX_BITS][3];     // twice the X coefficient of tile bit m in three floats
 };
 
 struct ZvFF {
     using S = double2;
     using V = ffp;
     static __device__ __forceinline__ V split(S a) { return to_ffp(a); }
-    // the split keeps neither magnitudes past the float range nor infinities and NaN
     // place of a tile index in shared memory: each arrangement of k_zzx_energy reads 8 different
     // 16-byte banks per phase
     static __device__ __forceinline__ unsigned place(unsigned x) { return x ^ ((x >> 3) & 7u); }
+    // the split keeps neither magnitudes past the float range nor infinities and NaN
     static __device__ __forceinline__ bool too_large(S a) {
         constexpr int most = (1023 + 40) << 20;
         return (__double2hiint(a.x) & 0x7FFFFFFF) >= most || (__double2hiint(a.y) & 0x7FFFFFFF) >= most;
@@ -136,14 +136,42 @@ __device__ __forceinline__ float2 ff_sign(float2 a, unsigned negative) {
     return negative & 1u ? make_float2(-a.x, -a.y) : a;
 }
 
-__device__ __forceinline__ double zzx_value(const PDot2& acc) {
-    u64 h, l;
-    acc.result(h, l);
-    float h0, h1, l0, l1;
-    up2(h, h0, h1);
-    up2(l, l0, l1);
-    return ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
-}
+// A thread's sum over its tiles, in three floats per lane (about 72 bits). A PDot2 carries the few
+// terms of one tile: its error sum is a float, and over equal terms its own rounding errors are equal
+// too (kept over all tiles, a register whose amplitudes depend on two wires came out 2.4e-11 off at 27
+// qubits of complex128 and 7.6e-11 of complex64; now 7e-15 and 4e-15, the f64 kernel 5e-15 and 1.7e-14).
+// Energy calls: complex128 24 qubits 385 -> 444 us, 30 qubits 26.2 -> 30.9 ms; complex64 30 qubits 12.6 ->
+// 13.1 ms.
+struct ZzxTotal {
+    u64 a, b, c;
+    __device__ __forceinline__ void clear() { a = b = c = 0; }
+    static __device__ __forceinline__ u64 two_sum(u64& s, u64 x) {  // s += x, the rounding error
+        const u64 t = padd(s, x), bb = psub(t, s);
+        const u64 e = padd(psub(s, psub(t, bb)), psub(x, bb));
+        s = t;
+        return e;
+    }
+    __device__ __forceinline__ void add(u64 h, u64 l) {
+        const u64 e = two_sum(a, h), e2 = two_sum(b, l), e3 = two_sum(b, e);
+        c = padd(c, padd(e2, e3));
+    }
+    __device__ __forceinline__ void add(const PDot2& d) { add(d.s, d.en ^ ZZX_SIGNS); }
+    // += w * d
+    __device__ __forceinline__ void add(const PDot2& d, const u64* w) {
+        const u64 p = pmul(w[0], d.s);
+        u64 r = pfma(w[0], d.s, p ^ ZZX_SIGNS);
+        r = pfma(w[1], d.s, r);
+        r = pfma(w[2], d.s, r);
+        add(p, pfma(w[0] ^ ZZX_SIGNS, d.en, r));
+    }
+    __device__ __forceinline__ double value() const {
+        float x[2], y[2], z[2];
+        up2(a, x[0], x[1]);
+        up2(b, y[0], y[1]);
+        up2(c, z[0], z[1]);
+        return ((double)x[0] + (double)x[1]) + (((double)y[0] + (double)y[1]) + ((double)z[0] + (double)z[1]));
+    }
+};
 
 // Amplitude of tile index t + 256 j of tile g: base + j * step.
 template <bool FIRST>
@@ -239,8 +267,9 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
     const unsigned t = threadIdx.x;
     if (FIRST) diag.tables(p, t);
     bool large = false;
-    PDot2 acc, nrm;
-    acc.s = acc.en = nrm.s = nrm.en = 0;
+    ZzxTotal energy, norm;
+    energy.clear();
+    norm.clear();
     typename P::S raw[ZZX_REGS];
     auto load = [&](uint64_t g) {
         uint64_t base, step;
@@ -272,6 +301,8 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
         __syncthreads();
         // (a pass that takes all bits of its tile, as all but the last do, tests none of them)
         auto work = [&](auto every) {
+            PDot2 acc, nrm;
+            acc.s = acc.en = nrm.s = nrm.en = 0;
 #pragma unroll
             for (int j = 0; j < ZZX_REGS; ++j) {
                 typename P::Sum s;
@@ -300,6 +331,8 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
                     }
                 }
             }
+            energy.add(acc);
+            if constexpr (FIRST) norm.add(nrm);
         };
         if constexpr (FIRST) {
             work(std::true_type{});
@@ -308,16 +341,17 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
             else work(std::false_type{});
         }
     }
-    zzx_sums<FIRST>(zzx_value(acc), FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0, partial);
+    zzx_sums<FIRST>(energy.value(), FIRST ? (large ? CUDART_INF : norm.value()) : 0.0, partial);
 }
 
 // The energy alone, complex128: the X term of bit m is 2 c_m sum Re conj(psi[x]) psi[x ^ 2^m] over the pairs,
 // one product per pair where H psi takes two per amplitude (half the operations), summed per bit
-// and weighted once per thread in f64. Three bits at a time lie in a thread's registers: the tile
+// over the tile and then weighted. Three bits at a time lie in a thread's registers: the tile
 // is written to shared memory once and read in three more arrangements (two in a later pass), 24
-// reads of an amplitude per thread instead of one per bit. Energy call: 24 qubits 520 -> 382 us, 30
-// qubits 38.0 -> 26.1 ms (8.9 of them the reads at HBM speed; L2 prefetches of the next tile cost 4).
-// Not for complex64, whose H psi takes one operation per amplitude and bit (18.1 against 12.6 ms).
+// reads of an amplitude per thread instead of one per bit. Energy call, k_zzx /
+// k_zzx_energy: 24 qubits 564 / 444 us, 30 qubits 41.0 / 30.9 ms (8.9 of them the reads at HBM speed; L2
+// prefetches of the next tile cost 4). Not for complex64, whose H psi takes one operation per
+// amplitude and bit (30 qubits 18.1 against 12.6 ms before the sums in three floats).
 template <bool FIRST>
 __global__ void __launch_bounds__(ZZX_THREADS, 2)
 k_zzx_energy(const double2* __restrict__ psi, const __grid_constant__ ZzxParams p,
@@ -329,10 +363,9 @@ k_zzx_energy(const double2* __restrict__ psi, const __grid_constant__ ZzxParams 
     const unsigned t = threadIdx.x;
     if (FIRST) diag.tables(p, t);
     bool large = false;
-    PDot2 acc, nrm, bit[ZZX_BITS];
-    acc.s = acc.en = nrm.s = nrm.en = 0;
-#pragma unroll
-    for (int m = 0; m < ZZX_BITS; ++m) bit[m].s = bit[m].en = 0;
+    ZzxTotal energy, norm;
+    energy.clear();
+    norm.clear();
     const unsigned at0 = P::place(t), at1 = P::place((t & 31u) | ((t >> 5) << 8)),
                    at2 = P::place((t & 3u) | ((t >> 2) << 5)), at3 = P::place(t << 3);
     for (uint64_t g = blockIdx.x; g < p.ntiles; g += gridDim.x) {
@@ -353,6 +386,8 @@ k_zzx_energy(const double2* __restrict__ psi, const __grid_constant__ ZzxParams 
         if (FIRST) diag.above(p, g, t);
         __syncthreads();
         if constexpr (FIRST) {
+            PDot2 acc, nrm;
+            acc.s = acc.en = nrm.s = nrm.en = 0;
 #pragma unroll
             for (int j = 0; j < ZZX_REGS; ++j) {
                 typename P::Sum s;
@@ -360,41 +395,38 @@ k_zzx_energy(const double2* __restrict__ psi, const __grid_constant__ ZzxParams 
                 P::term(acc, v[j], s.result());
                 P::term(nrm, v[j], v[j]);
             }
+            energy.add(acc);
+            norm.add(nrm);
         }
-        // the pairs of tile bits m0 .. m0 + 2, in register bits 0 .. 2
-        auto pairs = [&](auto m0) {
+        // the pairs of tile bits m0 .. m0 + COUNT - 1, in register bits 0 ..
+        auto pairs = [&](auto m0, auto count) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < decltype(count)::value; ++k) {
                 constexpr int M0 = decltype(m0)::value;
                 if (!((p.terms >> (M0 + k)) & 1u)) continue;
+                PDot2 bit;
+                bit.s = bit.en = 0;
 #pragma unroll
                 for (int j = 0; j < ZZX_REGS; ++j)
-                    if (!(j & (1 << k))) P::term(bit[M0 + k], v[j], v[j | (1 << k)]);
+                    if (!(j & (1 << k))) P::term(bit, v[j], v[j | (1 << k)]);
+                energy.add(bit, p.twice[M0 + k]);
             }
         };
-        pairs(std::integral_constant<int, 8>{});
+        constexpr std::integral_constant<int, 3> three{};
+        pairs(std::integral_constant<int, 8>{}, three);
 #pragma unroll
         for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at1 ^ P::place(j << 5)];
-        pairs(std::integral_constant<int, 5>{});
+        pairs(std::integral_constant<int, 5>{}, three);
 #pragma unroll
         for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at2 ^ P::place(j << 2)];
-        pairs(std::integral_constant<int, 2>{});
+        pairs(std::integral_constant<int, 2>{}, three);
         if constexpr (FIRST) {
 #pragma unroll
             for (int j = 0; j < ZZX_REGS; ++j) v[j] = tile[at3 ^ P::place(j)];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (!((p.terms >> k) & 1u)) continue;
-#pragma unroll
-                for (int j = 0; j < ZZX_REGS; ++j)
-                    if (!(j & (1 << k))) P::term(bit[k], v[j], v[j | (1 << k)]);
-            }
+            pairs(std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
         }
     }
-    double e = FIRST ? zzx_value(acc) : 0.0;
-#pragma unroll
-    for (int m = FIRST ? 0 : ZZX_LOW; m < ZZX_BITS; ++m) e = fma(p.twice[m], zzx_value(bit[m]), e);
-    zzx_sums<FIRST>(e, FIRST ? (large ? CUDART_INF : zzx_value(nrm)) : 0.0, partial);
+    zzx_sums<FIRST>(energy.value(), FIRST ? (large ? CUDART_INF : norm.value()) : 0.0, partial);
 }
 
 // out[r] = sum of row r (nb values each): one warp per row, fixed order
@@ -456,7 +488,11 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
             const int bit = first + m - low;
             if (bit < done || bit >= n) continue;
             p.terms |= 1u << m;
-            p.twice[m] = 2.0 * H.b[n - 1 - bit];
+            const double w = 2.0 * H.b[n - 1 - bit];
+            const float wh = (float)w, wl = (float)(w - (double)wh);
+            p.twice[m][0] = both(wh);
+            p.twice[m][1] = both(wl);
+            p.twice[m][2] = both((float)((w - (double)wh) - (double)wl));
             const float2 c = coef_pair(H.b[n - 1 - bit]);
             p.x[m].c[0] = both(c.x);
             p.x[m].c[1] = both(c.y);

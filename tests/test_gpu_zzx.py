@@ -11,6 +11,7 @@ import pytest
 from quantr_gb300 import _native as nat
 from quantr_gb300 import gradients as GR
 from quantr_gb300 import workloads as W
+from quantr_gb300.program import ProgramBuilder
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +86,57 @@ def test_gradient_through_the_tiled_vectors(n, precision):
     tol = 1e-11 if precision == nat.QGPU_C128 else 1e-4
     assert abs(e - re) <= tol
     assert np.max(np.abs(g - rg)) <= tol
+
+
+# 17, 20: k_zzx of an energy; 22, 25, 27: k_zzx_energy, one, 54 and 216 tiles a CTA
+@pytest.mark.parametrize("n", [17, 20, 22, 25, 27])
+@pytest.mark.parametrize("precision", [nat.QGPU_C128, nat.QGPU_C64])
+def test_energy_of_registers_with_few_values(n, precision):
+    """Amplitudes that depend on the last two wires alone: every thread adds up equal terms, whose
+    rounding errors do not cancel. Bar: of a term, the amplitudes' splits (2 * 2^-49), the product
+    of their low parts (2^-48), and the errors of a tile's up to 8 sums (8 * 2^-24 * 2^-25), then sums
+    over the tiles in triples of floats: 4e-14 of it (complex64: the tile's sums alone, of amplitudes
+    and neighbours that are exact with one coefficient of 1)."""
+    r = np.random.default_rng(n)
+    for _ in range(3 if n < 25 else 1):
+        c = r.uniform(0.3, 1.0, 4) * 2.0 ** (-n / 2)
+        if precision == nat.QGPU_C64:
+            c = c.astype(np.float32).astype(np.float64)
+        h = nat.Handle(n, precision)
+        psi = np.empty((1 << (n - 2), 4), np.complex128)
+        psi[:] = c
+        h.upload(psi.reshape(-1))
+        del psi
+        sq = c * c
+        N = 2.0 ** (n - 2)
+        one, zero = np.zeros(n), np.zeros(n)
+        for wire in (0, n // 2, n - 3):  # X on a wire in |+>: the norm
+            one[:] = 0.0
+            one[wire] = 1.0
+            want = N * sq.sum()
+            assert abs(h.expectation_zzx(zero, one) - want) <= 4e-14 * want
+        one[:] = 0.0
+        one[n - 1] = 1.0
+        want = 2.0 * N * (c[0] * c[1] + c[2] * c[3])
+        assert abs(h.expectation_zzx(zero, one) - want) <= 4e-14 * want
+        one[:] = 0.0
+        one[n - 2] = 1.0  # ZZ of the last two wires
+        want = N * (sq[0] - sq[1] - sq[2] + sq[3])
+        assert abs(h.expectation_zzx(one, zero) - want) <= 4e-14 * N * sq.sum()
+        h.close()
+
+
+@pytest.mark.parametrize("n", [20, 25])
+def test_gradient_energy_of_registers_with_few_values(n):
+    """The same through H psi (energy_and_gradient): |+> on all wires and one Ry, whose energy is known;
+    divided by the register's norm, the state's own rounding leaves 2^-48 per gate and wire."""
+    b = ProgramBuilder(n)
+    for w in range(n):
+        b.add("H", w)
+    b.add("Ry", n - 1, (), param=0.3)
+    prog = b.build()
+    h = nat.Handle(n)
+    x = np.random.default_rng(n).uniform(0.5, 1.0, n)
+    e, _ = GR.energy_and_gradient(h, prog, np.zeros(n), x)
+    want = x[:-1].sum() + x[-1] * np.cos(0.3)
+    assert abs(e / h.norm() - want) <= 1e-13 * x.sum()
