@@ -30,11 +30,6 @@ constexpr int ZZX_BITS = 11;    // tile bits: 8 in the thread index, 3 in a thre
 constexpr int ZZX_LOW = 3;      // low bits of the tiles of the later passes
 constexpr int ZZX_REGS = 8;     // amplitudes per thread
 constexpr int ZZX_FIELD = ZZX_BITS - ZZX_LOW;
-// Smallest complex128 register whose energy alone is taken pair by pair (k_zzx_energy: two CTAs per
-// SM, so fewer tiles leave SMs idle): energy call, k_zzx / k_zzx_energy, at 20 qubits 72 / 85 us, at
-// 21 96 / 99, at 22 150 / 133, at 24 541 / 382.
-constexpr int ZZX_PAIRS_QUBITS = 22;
-
 constexpr u64 ZZX_SIGNS = 0x8000000080000000ull;  // both lanes negated
 
 // Coefficients as the packed operands of a Dot2 term (hi, lo, -hi, -lo), both lanes alike.
@@ -254,7 +249,7 @@ __device__ __forceinline__ void zzx_sums(double e, double q, double* __restrict_
 // (above the 3 lowest). psi's copy goes to phi and H psi to lam, both in the sweep's layout
 // (P::put); later passes read phi and add to lam. Without VEC only the energy is formed (complex64;
 // the next tile's amplitudes are loaded while this one is worked on: 14.7 -> 12.6 ms at 30 qubits,
-// with a pass that takes all its bits not testing each; and complex128 below 22 qubits). partial[blockIdx] gets the
+// with a pass that takes all its bits not testing each). partial[blockIdx] gets the
 // pass's share of Re <psi|H psi>, and with FIRST partial[gridDim + blockIdx] that of <psi|psi>.
 template <class P, bool FIRST, bool VEC>
 __global__ void __launch_bounds__(ZZX_THREADS, sizeof(typename P::S) == 8 ? (VEC ? 4 : 2) : FIRST ? 2 : 3)
@@ -349,7 +344,7 @@ k_zzx(const typename P::S* __restrict__ psi, typename P::S* __restrict__ phi,
 // over the tile and then weighted. Three bits at a time lie in a thread's registers: the tile
 // is written to shared memory once and read in three more arrangements (two in a later pass), 24
 // reads of an amplitude per thread instead of one per bit. Energy call, k_zzx /
-// k_zzx_energy: 24 qubits 564 / 444 us, 30 qubits 41.0 / 30.9 ms (8.9 of them the reads at HBM speed; L2
+// k_zzx_energy: 17 qubits 38.5 / 36.0 us, 20 73 / 64, 24 564 / 444, 30 qubits 41.0 / 30.9 ms (8.9 of them the reads at HBM speed; L2
 // prefetches of the next tile cost 4). Not for complex64, whose H psi takes one operation per
 // amplitude and bit (30 qubits 18.1 against 12.6 ms before the sums in three floats).
 template <bool FIRST>
@@ -456,10 +451,9 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
     static_assert(1 + (MAX_HAM_QUBITS - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD + 1 <= 8, "row sums");
     const int npass = 1 + (n - ZZX_BITS + ZZX_FIELD - 1) / ZZX_FIELD;
     int occ = 0;
-    bool pairs = false;  // k_zzx_energy
-    if constexpr (!VEC && sizeof(typename P::S) == 16) pairs = n >= ZZX_PAIRS_QUBITS;
+    constexpr bool pairs = !VEC && sizeof(typename P::S) == 16;  // k_zzx_energy
     cudaError_t e;
-    if (pairs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx_energy<true>, ZZX_THREADS, 0);
+    if constexpr (pairs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx_energy<true>, ZZX_THREADS, 0);
     else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_zzx<P, true, VEC>, ZZX_THREADS, 0);
     if (e != cudaSuccess || occ < 1) occ = 1;
     const uint64_t ntiles = h->dim >> ZZX_BITS;
@@ -501,11 +495,9 @@ static int run_zzx(qgpu_handle* h, const typename P::S* psi, typename P::S* phi,
         }
         done = first + ZZX_BITS - low;
         double* row = partial + (pass == 0 ? 0 : (size_t)(pass + 1) * nb);
-        if (pairs) {
-            if constexpr (sizeof(typename P::S) == 16) {
-                if (pass == 0) k_zzx_energy<true><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
-                else k_zzx_energy<false><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
-            }
+        if constexpr (pairs) {
+            if (pass == 0) k_zzx_energy<true><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
+            else k_zzx_energy<false><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, p, row);
         } else {
             if (pass == 0) k_zzx<P, true, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, row);
             else k_zzx<P, false, VEC><<<nb, ZZX_THREADS, 0, h->stream>>>(psi, phi, lam, p, row);
