@@ -4,7 +4,7 @@
 // A CTA stages a tile of both vectors in shared memory: the 2^K amplitudes that share every bit
 // outside the pass's K tile bits (the wires' bits and the lowest other bits, so that runs of
 // consecutive amplitudes load together). A wire's undo is exp(i a) D2 R D1 with D = diag(1, rho) and
-// R real (adj_frame, plan.cpp), the phase exp(i a) common to both vectors and left out. Per tile:
+// R real (pauli_frame, plan.cpp), the phase exp(i a) common to both vectors and left out. Per tile:
 //   load   q = Im(conj(l) f) of every amplitude (the wires' Z sums and the -I sum are signed sums
 //          of it: the sign of tile bits held in the thread index is applied once, at the end),
 //          then D1 of all wires at once as one factor per amplitude;
@@ -173,8 +173,13 @@ struct AgFF {
     };
 };
 
-// Z and -I sums over all tiles of a thread's products, lane 0 - lane 1: one Dot2 per register index.
+// Z and -I sums of a thread's products, lane 0 - lane 1: one Dot2 per register index, folded every
+// FLUSH tiles into sums of three floats. Kept over all tiles the Dot2's float error sum rounds more and
+// more, and where amplitudes take few values alike in every thread (27 qubits: a gradient off by
+// 4e-13 of sum|b|, now 3e-15). The 20-qubit gradient 3.25 -> 3.30 ms; three floats per product and register
+// index instead 3.64 ms, for the registers.
 struct AgZFF {
+    static constexpr int FLUSH = 16;
     AgFF::Sum z[AG_PER];
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -185,12 +190,10 @@ struct AgZFF {
         z[j].add(l, AgFF::neg(l), AgFF::swap(f));
     }
     __device__ __forceinline__ void end_tile() {}
-    // the sum (m < 0), or signed by bit m of the register index
-    __device__ __forceinline__ AgF3 value(int m) const {
-        AgF3 v = {0.f, 0.f, 0.f};
+    // v += the sum (m < 0), or the sum signed by bit m of the register index
+    __device__ __forceinline__ void value(int m, AgF3& v) const {
 #pragma unroll
         for (int j = 0; j < AG_PER; ++j) z[j].lanes3(v, m >= 0 && ((j >> m) & 1));
-        return v;
     }
 };
 
@@ -267,6 +270,7 @@ struct AgF32 {
 
 // The same with f32 sums of one tile's products, the sum and the three signed sums.
 struct AgZF32 {
+    static constexpr int FLUSH = 0;  // (never: the error sums' rounding lies far below the f32 products')
     AgF32::Sum z[4];
     u64 q[4];
     __device__ __forceinline__ void clear() {
@@ -284,11 +288,7 @@ struct AgZF32 {
 #pragma unroll
         for (int k = 0; k < 4; ++k) z[k].add_tile(q[k]);
     }
-    __device__ __forceinline__ AgF3 value(int m) const {
-        AgF3 v = {0.f, 0.f, 0.f};
-        z[m < 0 ? 3 : m].lanes3(v, false);
-        return v;
-    }
+    __device__ __forceinline__ void value(int m, AgF3& v) const { z[m < 0 ? 3 : m].lanes3(v, false); }
 };
 template <class P>
 struct AgZ {
@@ -365,6 +365,23 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
         red[i] = make_float2(0.f, 0.f);
     typename AgZ<P>::type z;
     z.clear();
+    // sums up to the last flush (all, register bits 0..2; indexed in a loop: they lie in local memory)
+    constexpr int FLUSH = AgZ<P>::type::FLUSH;
+    AgF3 ztot[AG_RBITS + 1];
+    if constexpr (FLUSH > 0) {
+#pragma unroll 1
+        for (int k = 0; k <= AG_RBITS; ++k) ztot[k] = {0.f, 0.f, 0.f};
+    }
+    auto flush = [&]() {
+#pragma unroll 1
+        for (int k = 0; k <= AG_RBITS; ++k) {
+            AgF3 v = ztot[k];
+            z.value(k - 1, v);
+            ztot[k] = v;
+        }
+        z.clear();
+    };
+    int tiles = 0;
     if (t >= T && t < (1 << p.tile)) sf[ag_slot(t)] = sl[ag_slot(t)] = V{};
     __syncthreads();
     for (uint64_t g = blockIdx.x; g < p.ngroups; g += gridDim.x) {
@@ -387,6 +404,12 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
                 sl[ag_slot(t + j * AG_THREADS)] = l;
             }
             z.end_tile();
+        }
+        if constexpr (FLUSH > 0) {
+            if (p.zsum && ++tiles == FLUSH) {
+                flush();
+                tiles = 0;
+            }
         }
         __syncthreads();
         if (t < T && g + gridDim.x < p.ngroups) {  // the next tile heads for L2
@@ -495,8 +518,18 @@ k_adj_group(typename P::S* __restrict__ phi, typename P::S* __restrict__ lam,
     __syncthreads();
     AgF3* zs = reinterpret_cast<AgF3*>(smem);  // [all, register bits 0..2][thread]
     if (p.zsum) {
+        if constexpr (FLUSH > 0) {
+            flush();
+#pragma unroll 1
+            for (int k = 0; k <= AG_RBITS; ++k) zs[k * AG_THREADS + t] = ztot[k];
+        } else {
 #pragma unroll
-        for (int k = 0; k <= AG_RBITS; ++k) zs[k * AG_THREADS + t] = z.value(k - 1);
+            for (int k = 0; k <= AG_RBITS; ++k) {
+                AgF3 v = {0.f, 0.f, 0.f};
+                z.value(k - 1, v);
+                zs[k * AG_THREADS + t] = v;
+            }
+        }
     }
     __syncthreads();
     const int lane = t & 31;

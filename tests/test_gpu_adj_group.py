@@ -59,3 +59,26 @@ def test_grouped_passes_against_the_f64_sweep(monkeypatch, n, run, precision):
     tol = 1e-11 if precision == nat.QGPU_C128 else 1e-4
     assert abs(e - re) <= tol
     assert np.max(np.abs(g - rg)) <= tol
+
+
+@pytest.mark.parametrize("n", [21, 27])
+def test_z_sums_of_registers_with_few_values(n):
+    """Phases on low wires alone and no ZZ terms: a thread's products over its tiles are equal, and so
+    are their rounding errors. The Z sums (Rz) and the -I sum (Phase) against the f64 sweep. Bar, in
+    units of S = sum|x|: 2^-47 for a product of two float pairs, and the rounding of both vectors,
+    2^-49 for each of the n + 5 gates each way, which equal amplitudes share: 1.2e-13 for n = 27, of which
+    1e-13 is allowed."""
+    b = ProgramBuilder(n)
+    for w in range(n):
+        b.add("H", w)
+    b.add("Ry", n - 1, (), param=0.3)
+    b.add("Rz", n - 1, (), param=0.7)
+    b.add("Phase", n - 1, (), param=0.4)
+    b.add("Rz", n - 2, (), param=0.2)
+    b.add("Rz", n - 5, (), param=-0.5)
+    prog = b.build()
+    x = np.random.default_rng(n).uniform(0.5, 1.0, n)
+    e, g = GR.energy_and_gradient(nat.Handle(n), prog, np.zeros(n), x)
+    re, rg = GR.energy_and_gradient(nat.Handle(n, nat.QGPU_C128, nat.QGPU_MODE_F64), prog, np.zeros(n), x)
+    assert abs(e - re) <= 1e-13 * x.sum()
+    assert np.max(np.abs(g - rg)) <= 1e-13 * x.sum()
