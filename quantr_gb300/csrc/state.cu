@@ -143,8 +143,9 @@ __global__ void k_reduce_partial(const T* __restrict__ s, uint64_t dim, uint64_t
 
 // sum |a|^2 of a complex64 register: error-free products and sums in packed f32 over 32 amplitudes at
 // a time, then f64 (the per-amplitude conversions and multiply-adds kept the FP64 pipe busy: 7.7 ms at
-// 30 qubits against HBM's 1.3). Over 32 amplitudes the error sum stays below 2^-43 of the chunk,
-// of either sign, so that over a register it vanishes against f64 rounding.
+// 30 qubits against HBM's 1.3). Both rounding errors, of the square and of the sum, go to a second sum
+// and its errors to a third, so that a chunk is exact to 2^-60: with the second alone, equal amplitudes
+// made equal errors in every chunk, up to 2^-42 of the norm (30 qubits: 1.37 -> 1.52 ms).
 __global__ void __launch_bounds__(RED_THREADS) k_norm_f32(const float4* __restrict__ s, uint64_t pairs,
                                                           uint64_t per_block, double2* __restrict__ partial) {
     __shared__ double sh[RED_THREADS];
@@ -153,40 +154,48 @@ __global__ void __launch_bounds__(RED_THREADS) k_norm_f32(const float4* __restri
     if (end > pairs) end = pairs;
     constexpr int CHUNK = 16;  // amplitude pairs
     double total = 0.0;
-    auto add = [](u64& sum, u64& err, float x, float y) {
-        const u64 v = p2(x, y), p = pmul(v, v);
-        const u64 r = pfma(v, v, p ^ 0x8000000080000000ull);
-        const u64 t = padd(sum, p);
-        const u64 bb = psub(t, sum);
-        err = padd(err, padd(padd(psub(sum, psub(t, bb)), psub(p, bb)), r));
-        sum = t;
-    };
-    auto flush = [&](u64 sum, u64 err) {
-        float a, b, c, d;
-        up2(sum, a, b);
-        up2(err, c, d);
-        total += ((double)a + (double)b) + ((double)c + (double)d);
+    struct Chunk {
+        u64 sum = 0, err = 0, rest = 0;
+        static __device__ __forceinline__ u64 two_sum(u64& a, u64 x) {  // a += x, the rounding error
+            const u64 t = padd(a, x), bb = psub(t, a);
+            const u64 e = padd(psub(a, psub(t, bb)), psub(x, bb));
+            a = t;
+            return e;
+        }
+        __device__ __forceinline__ void add(float x, float y) {
+            const u64 v = p2(x, y), p = pmul(v, v);
+            const u64 r = pfma(v, v, p ^ 0x8000000080000000ull);
+            const u64 q = two_sum(sum, p), e = two_sum(err, q), d = two_sum(err, r);
+            rest = padd(rest, padd(e, d));
+        }
+        __device__ __forceinline__ double value() const {
+            float a, b, c, d, e, f;
+            up2(sum, a, b);
+            up2(err, c, d);
+            up2(rest, e, f);
+            return ((double)a + (double)b) + (((double)c + (double)d) + (double)(e + f));
+        }
     };
     uint64_t i = begin + threadIdx.x;
     for (; i + (CHUNK - 1) * (uint64_t)RED_THREADS < end; i += CHUNK * (uint64_t)RED_THREADS) {
         float4 v[CHUNK];
 #pragma unroll
         for (int k = 0; k < CHUNK; ++k) v[k] = s[i + k * (uint64_t)RED_THREADS];
-        u64 sum = 0, err = 0;
+        Chunk c;
 #pragma unroll
         for (int k = 0; k < CHUNK; ++k) {
-            add(sum, err, v[k].x, v[k].y);
-            add(sum, err, v[k].z, v[k].w);
+            c.add(v[k].x, v[k].y);
+            c.add(v[k].z, v[k].w);
         }
-        flush(sum, err);
+        total += c.value();
     }
-    u64 sum = 0, err = 0;
+    Chunk c;
     for (; i < end; i += RED_THREADS) {  // fewer than a chunk
         const float4 v = s[i];
-        add(sum, err, v.x, v.y);
-        add(sum, err, v.z, v.w);
+        c.add(v.x, v.y);
+        c.add(v.z, v.w);
     }
-    flush(sum, err);
+    total += c.value();
     sh[threadIdx.x] = total;
     __syncthreads();
     for (int w = RED_THREADS / 2; w > 0; w >>= 1) {

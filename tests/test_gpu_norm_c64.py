@@ -29,3 +29,17 @@ def test_norm_of_infinite_and_nan_amplitudes(gpu_lib):
         h = nat.Handle(17, nat.QGPU_C64)
         h.upload(psi)
         assert not np.isfinite(h.norm())
+
+
+@pytest.mark.parametrize("n", [16, 17, 20, 24])
+def test_norm_of_equal_amplitudes(gpu_lib, n):
+    """Equal amplitudes make equal rounding errors in every chunk: nothing cancels over the register.
+    Bar: the squares are exact and a thread's 32 of them are summed to 2^-60, then f64 sums of at
+    most 2 chunks per thread, 8 and 5 + 8 levels of a tree, 2^-53 each: 23 * 2^-53 < 4e-15."""
+    r = np.random.default_rng(n)
+    for c in r.uniform(0.5, 1.0, 4 if n == 24 else 16):
+        v = np.float32(c * 2.0 ** (-n / 2))
+        h = nat.Handle(n, nat.QGPU_C64)
+        h.upload(np.full(1 << n, complex(float(v), 0.0)))
+        assert abs(h.norm() / (float(v) ** 2 * 2.0 ** n) - 1.0) <= 4e-15
+        h.close()
