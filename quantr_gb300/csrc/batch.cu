@@ -15,11 +15,11 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "internal.cuh"
 #include "plan.h"
+#include "workers.h"
 
 namespace qgpu {
 
@@ -706,7 +706,7 @@ extern "C" int qgpu_batch_run(const qgpu_batch_item* items, size_t n_items, cons
     QGPU_CUDA(cudaGetDevice(&dev));
     cudaDeviceProp prop;
     QGPU_CUDA(cudaGetDeviceProperties(&prop, dev));
-    // ---- small circuits: persistent launches from a CUDA graph, beside the large ones
+    // ---- small circuits: persistent launches, beside the large ones
     SmallBatch sb;
     if (!small.empty()) {
         sb.items = small;
@@ -729,6 +729,18 @@ extern "C" int qgpu_batch_run(const qgpu_batch_item* items, size_t n_items, cons
     std::atomic<int> first_err{QGPU_OK};
     std::string err_msg;
     std::mutex err_mu;
+    auto failed = [&](int st, const std::string& msg) {
+        int expect = QGPU_OK;
+        if (first_err.compare_exchange_strong(expect, st)) {
+            std::lock_guard<std::mutex> lk(err_mu);
+            err_msg = msg;
+        }
+    };
+    auto enter = [&]() {  // handles are created on the thread's current device
+        const cudaError_t e = cudaSetDevice(dev);
+        if (e != cudaSuccess) failed(cuda_fail(e, "cudaSetDevice"), qgpu_last_error());
+        return e == cudaSuccess;
+    };
     auto work = [&]() {
         qgpu_handle* h = nullptr;
         for (;;) {
@@ -753,20 +765,13 @@ extern "C" int qgpu_batch_run(const qgpu_batch_item* items, size_t n_items, cons
                                        obs + it.obs_offset, obs + it.obs_offset + it.n_qubits,
                                        &energies[i], grads + it.grad_offset);
             if (st != QGPU_OK) {
-                int expect = QGPU_OK;
-                if (first_err.compare_exchange_strong(expect, st)) {
-                    std::lock_guard<std::mutex> lk(err_mu);
-                    err_msg = qgpu_last_error();
-                }
+                failed(st, qgpu_last_error());
                 break;
             }
         }
         if (h) qgpu_destroy(h);
     };
-    std::vector<std::thread> pool;
-    for (int w = 1; w < workers; ++w) pool.emplace_back(work);
-    work();
-    for (auto& t : pool) t.join();
+    run_workers(workers, enter, work);
     if (first_err.load() != QGPU_OK) return fail(first_err.load(), err_msg);
     return small.empty() ? QGPU_OK : sb.finish(items, energies, grads);
 }
