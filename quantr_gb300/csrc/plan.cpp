@@ -1876,6 +1876,9 @@ PauliFrame pauli_frame(PauliRun* run) {
     const std::array<cd, 4>& m = run->undo;  // m00 m01 m10 m11
     PauliFrame f;
     auto unit = [](cd z) { return z / std::abs(z); };
+    // entries this small (Rx of 1e-310) change no f64 result, but a product of one with another entry
+    // is a subnormal number of few digits, or 0, and has no direction to take
+    auto none = [](cd z) { return std::abs(z) < 1e-150; };
     if (!run->framed) {
         f.c = std::abs(m[0]);
         f.s = std::abs(m[1]);
@@ -1890,11 +1893,11 @@ PauliFrame pauli_frame(PauliRun* run) {
             f.rho2 = 1.0;
             if (f.c < 0.0) f.c = 1.0;
         }
-    } else if (m[1] == cd(0.0, 0.0)) {  // diagonal
+    } else if (none(m[1]) || none(m[2])) {  // diagonal
         f.c = 1.0;
         f.s = 0.0;
         f.rho1 = unit(m[3] / m[0]);
-    } else if (m[0] == cd(0.0, 0.0)) {  // e^{i a} [[0, -rho1], [1, 0]]
+    } else if (none(m[0])) {  // e^{i a} [[0, -rho1], [1, 0]]
         f.c = 0.0;
         f.s = 1.0;
         f.rho1 = unit(-m[1] / m[2]);
