@@ -97,3 +97,25 @@ def test_digit_passes_with_measurement_and_norm(oracle):
     same = h.measure_uniforms(u) == oracle.measure_uniforms(h.download(), u)
     assert same.sum() >= 1998
     h.close()
+
+
+@pytest.mark.parametrize("n,least", [(20, 20), (22, 20), (24, None)])
+def test_digit_passes_at_large_sizes(monkeypatch, oracle, n, least):
+    """From the smallest registers whose digits were the default, and the default's own threshold; at
+    24 qubits against the f64 mode (itself within 1e-13 of the oracle at 20 and 22 qubits)."""
+    if least is None:
+        monkeypatch.delenv("QGPU_DIGITS_MIN_QUBITS")
+    else:
+        monkeypatch.setenv("QGPU_DIGITS_MIN_QUBITS", str(least))
+    prog = W.brickwork_qft(n=n, layers=8, seed=n)
+    if n < 24:
+        ref = oracle.simulate(prog, engine=oracle.DENSE_PAR)
+    else:
+        h = nat.Handle(n, nat.QGPU_C128, nat.QGPU_MODE_F64)
+        h.apply(prog.ops, prog.mats, prog.none)
+        ref = h.download()
+        h.close()
+    out, prof = _run(prog, profile=True)
+    assert "k_dg2" in prof and "k_dg_from" in prof and "k_dg_to" in prof, prof
+    assert not any(k.startswith("k_pair2<") for k in prof), prof
+    assert np.max(np.abs(out - ref)) <= TOL
