@@ -133,50 +133,6 @@ k_adj_1q(double2* __restrict__ phi, double2* __restrict__ lam, uint64_t npairs,
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
-// The same sweep step for QGPU_MODE_FAST: the gradient term stays f64 (4 FMAs per pair on the
-// loaded doubles) while phi and lambda are updated with float-pair arithmetic (packed Dot2).
-struct AdjStepFF {
-    int t;
-    int gen;
-    u64 pk[32];  // ST_DENSE packed constants of V = U^dagger
-};
-
-__global__ void __launch_bounds__(ADJ_THREADS)
-k_adj_1q_ff(double2* __restrict__ phi, double2* __restrict__ lam, uint64_t npairs,
-            const __grid_constant__ AdjStepFF s, double* __restrict__ partial) {
-    __shared__ double sh[ADJ_THREADS];
-    double acc = 0.0;
-    for (uint64_t p = blockIdx.x * (uint64_t)ADJ_THREADS + threadIdx.x; p < npairs;
-         p += (uint64_t)gridDim.x * ADJ_THREADS) {
-        const uint64_t i0 = insert_zero(p, s.t), i1 = i0 | (1ull << s.t);
-        const double2 f0 = phi[i0], f1 = phi[i1], l0 = lam[i0], l1 = lam[i1];
-        switch (s.gen) {
-            case 1: acc += fma(l0.x, f1.y, -l0.y * f1.x) + fma(l1.x, f0.y, -l1.y * f0.x); break;
-            case 2: acc += fma(l1.x, f0.x, l1.y * f0.y) - fma(l0.x, f1.x, l0.y * f1.y); break;
-            case 3: acc += fma(l0.x, f0.y, -l0.y * f0.x) - fma(l1.x, f1.y, -l1.y * f1.x); break;
-            case 4: acc -= fma(l0.x, f0.y, -l0.y * f0.x) + fma(l1.x, f1.y, -l1.y * f1.x); break;
-            default: break;
-        }
-        ffp a = to_ffp(f0), b = to_ffp(f1);
-        ff_dense(a, b, s.pk);
-        phi[i0] = from_ffp(a);
-        phi[i1] = from_ffp(b);
-        a = to_ffp(l0);
-        b = to_ffp(l1);
-        ff_dense(a, b, s.pk);
-        lam[i0] = from_ffp(a);
-        lam[i1] = from_ffp(b);
-    }
-    if (!partial) return;
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = ADJ_THREADS / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
-}
-
 // ---------------------------------------------------------------------------------------------
 // k_adj_tile<K>: a run of single-wire gates of the reverse sweep, on up to K wires, in one pass.
 // Gates on different wires commute, so the run is regrouped wire by wire (each wire's gates in
@@ -761,16 +717,14 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
         std::vector<std::vector<size_t>> gates;
         by_wire(ops, run, h->n_qubits, &wires, &gates);
         run.clear();
-        // Pauli-sum passes take less arithmetic (one 2x2 update per vector per wire instead of
-        // one per gate) and win once the vectors live in HBM; with the vectors in L2 (up to 21
-        // qubits) the per-gate passes measured faster on GB300 (20 qubits: 6.39 against 6.68 ms;
-        // 24 qubits: 35.1 against 29.9 ms). Tuning knob QGPU_ADJ_PAULI: 0 / 1 forces either.
-        const char* pk = std::getenv("QGPU_ADJ_PAULI");  // read per call (tests force either)
-        const int pauli_knob = (pk && pk[0] == '0') ? 0 : (pk && pk[0] == '1') ? 1 : -1;
         // Grouped passes (adj_group.cu: the wires of a run in tiles of up to 10 bits, one pass per
-        // tile); QGPU_ADJ_GROUP=0 (read per call) selects one pass per wire. Measured on GB300
+        // tile). As second opinions for the tests, read per call: QGPU_ADJ_PAULI=0 one update per
+        // gate, QGPU_ADJ_GROUP=0 one pass per wire, with Pauli sums (QGPU_ADJ_PAULI=1, or from 22
+        // qubits, where they were the faster of the two) or per gate. Measured on GB300
         // (4-layer ansatz, energy + gradient, grouped against per-wire): 13 qubits 0.51 / 0.77 ms,
         // 20 qubits 1.46 / 2.54 ms, 24 qubits 16.9 / 26.2 ms, 25 qubits 33.8 / 52.6 ms.
+        const char* pk = std::getenv("QGPU_ADJ_PAULI");
+        const int pauli_knob = (pk && pk[0] == '0') ? 0 : (pk && pk[0] == '1') ? 1 : -1;
         const char* gk = std::getenv("QGPU_ADJ_GROUP");
         const bool group = pauli_knob != 0 && !(gk && gk[0] == '0');
         const bool pauli = pauli_knob >= 0 ? pauli_knob == 1 : h->n_qubits >= 22;
@@ -919,19 +873,8 @@ int qgpu_adjoint_grad(qgpu_handle* h, const qgpu_op* ops, size_t n_ops, const do
             terms[gi].emplace_back(nrows, 1.0);
             part = partial + (size_t)(nrows++) * nb;
         }
-        if (h->mode == QGPU_MODE_FAST) {
-            AdjStepFF f;
-            f.t = s.t;
-            f.gen = s.gen;
-            const cd v00(s.v[0], s.v[1]), v01(s.v[2], s.v[3]), v10(s.v[4], s.v[5]), v11(s.v[6], s.v[7]);
-            const DevStep ds = dense_step(v00, v01, v10, v11);
-            std::memcpy(f.pk, ds.pk, sizeof(f.pk));
-            k_adj_1q_ff<<<nb, ADJ_THREADS, 0, h->stream>>>(phi, lam, h->dim / 2, f, part);
-            QGPU_CHECK_LAUNCH("k_adj_1q_ff");
-        } else {
-            k_adj_1q<<<nb, ADJ_THREADS, 0, h->stream>>>(phi, lam, h->dim / 2, s, part);
-            QGPU_CHECK_LAUNCH("k_adj_1q");
-        }
+        k_adj_1q<<<nb, ADJ_THREADS, 0, h->stream>>>(phi, lam, h->dim / 2, s, part);
+        QGPU_CHECK_LAUNCH("k_adj_1q");
         h->launches++;
     }
     st = flush_run();
