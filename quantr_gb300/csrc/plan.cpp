@@ -1719,7 +1719,8 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
         }
         if (!own && opt.wide_bits > 0 && n >= opt.wide_table_qubits && i + 1 < steps.size() &&
             steps[i + 1].s.type == ST_TABLE && block_at[i] < 0) {
-            // rows of a Fourier transform: at least four tables at most two steps apart
+            // rows of a Fourier transform: at least two tables at most two steps apart (with four the
+            // transforms of complex64 on 5 and 6 qubits took 61 and 73 us in place of 57 and 66)
             int count = 0;
             size_t last = i;
             for (size_t q = i + 1; q < steps.size() && q <= last + 3 + (count == 0) && block_at[q] < 0; ++q)
@@ -1727,7 +1728,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
                     ++count;
                     last = q;
                 }
-            own = count >= 4;
+            own = count >= 2;
             if (own) j = last + 1;
         }
         if (!own) {

@@ -2049,9 +2049,10 @@ PlanOptions plan_options_for(const qgpu_handle* h) {
         o.wide_regs = ff ? WideFF::R : WideF32::R;
         o.wide_low = ff ? 2 : 3;
         o.wide_pairs = ff && dg_supported(h) ? 6 : 0;
-        // (Fourier transforms, wide against tile passes: complex128 at 19 qubits 205 / 243 us, at 20
-        // 378 / 317; complex64 at 18 qubits 216 / 166 us)
-        o.wide_table_qubits = ff ? 20 : 14;
+        // (Fourier transforms, call times with the rows in wide / in tile passes: complex128 at 7 qubits 70 /
+        // 74 us, 10 110 / 114, 11 155 / 146, 14 285 / 263, 18 449 / 402, 20 718 / 611; complex64 at 7 qubits 86 /
+        // 74 us, 9 119 / 96, 12 223 / 176, 14 328 / 257, 18 500 / 398)
+        o.wide_table_qubits = ff ? 11 : 0;
     }
     return o;
 }
