@@ -453,13 +453,17 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
     const bool whole = s.cm == 0 && (s.type == ST_REAL || s.type == ST_DENSE || s.type == ST_DENSE4);
     const bool third_kept = ff && s.type != ST_DENSE && s.type != ST_DENSE4;
     const bool given = s.given || (s.type == ST_DENSE4 && plan.pairs[ws.pair].given);
+    const bool phase = s.type == ST_PHASE && !s.unit && __builtin_popcountll(s.cm) == 1;
     double size = 0.0, exact = 0.0;  // sum of x^2 over the entries, and its rounding
-    for (cd z : e)
-        for (double x : {z.real(), z.imag()}) {
-            const double sq = x * x, sum = size + sq, b = sum - size;
-            exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
-            size = sum;
-        }
+    auto square = [&](double x) {
+        const double sq = x * x, sum = size + sq, b = sum - size;
+        exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
+        size = sum;
+    };
+    for (size_t k = 0; k < e.size() && (whole || phase); ++k) {
+        square(e[k].real());
+        if (s.type != ST_REAL) square(e[k].imag());
+    }
     // sum |e|^2 of a unitary d x d matrix is d (false for sizes that are not finite)
     const double d = given ? size : s.type == ST_DENSE4 ? 4.0 : s.type == ST_PHASE ? 1.0 : 2.0;
     const bool known = given ? size > 0.0 && size < HUGE_VAL : std::fabs(size - d) < 1e-12;
@@ -495,7 +499,7 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
         }
     }
     if (whole && known) *drift += 0.5 * (off + change) / d;
-    if (s.type == ST_PHASE && !s.unit && known && __builtin_popcountll(s.cm) == 1)
+    if (phase && known)
         *drift += 0.25 * (off + change) / d;  // (half the amplitudes)
     if (c.size() & 1) c.push_back(0);  // 16-byte aligned
     return c;
