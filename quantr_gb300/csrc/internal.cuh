@@ -82,7 +82,8 @@ struct qgpu_handle {
     // An upper bound on the register's largest |amplitude| (its norm, for a normalised state):
     // the digit passes scale their fixed point by it. Exact after set_zero (1), unknown after an
     // upload (computed on the device when a digit pass needs it), carried through plans (Custom
-    // gates multiply it by the Frobenius norm of their effective map).
+    // gates multiply it by the Frobenius norm of their effective map, as controlled 2x2s by the
+    // spectral norm, after which it counts as unknown unless they were unitary).
     double norm_bound = 1.0;
     bool norm_valid = true;
     uint64_t launches = 0;     // kernels launched on this handle (for benchmarking claims)

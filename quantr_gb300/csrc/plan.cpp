@@ -530,6 +530,14 @@ std::vector<AGate> fuse_pairs(const std::vector<AGate>& gates, int n, Plan* plan
     return out;
 }
 
+// The spectral norm of a 2x2, or 1 where that is more (infinite for entries that are not finite).
+double growth_of(const cd u[2][2]) {
+    double a = std::norm(u[0][0]) + std::norm(u[0][1]), b = std::norm(u[1][0]) + std::norm(u[1][1]);
+    const double c = std::abs(u[0][0] * std::conj(u[1][0]) + u[0][1] * std::conj(u[1][1]));
+    const double s = std::sqrt(0.5 * (a + b) + 0.5 * std::hypot(a - b, 2.0 * c));
+    return std::isfinite(s) ? std::max(1.0, s) : HUGE_VAL;
+}
+
 // Steps for a controlled 2x2 u on bit t under control mask cm.
 void emit_one(const AGate& g, std::vector<HStep>& out) {
     const cd u00 = g.u[0][0], u01 = g.u[0][1], u10 = g.u[1][0], u11 = g.u[1][1];
@@ -1278,6 +1286,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
     plan->wides.clear();
     plan->pairs.clear();
     plan->customs.clear();
+    plan->growth = 1.0;
     plan->table_ff.clear();
     plan->table_f64.clear();
     const int max_bits = std::max(1, std::min(opt.max_bits, std::min(n, MAX_TILE_BITS)));
@@ -1380,6 +1389,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
         a.support = support;
         for (int lo = 0; lo < 2; ++lo)
             for (int in = 0; in < 2; ++in) a.u[lo][in] = E[(call | in) * d + (call | lo)];
+        if (a.given) plan->growth *= growth_of(a.u);
         add_one(a, k == 1 && opt.merge_1q);
     }
 

@@ -214,6 +214,9 @@ struct Plan {
     std::vector<WidePass> wides;
     std::vector<PairBlock> pairs;      // fused pair blocks
     std::vector<LocalGate> customs;    // Custom gates, run by the group kernel
+    // How much the other Custom gates (controlled 2x2s, merged into steps) may grow an amplitude: the
+    // product of their spectral norms, each at least 1.
+    double growth = 1.0;
     std::vector<float> table_ff;       // TABLE entries as float pairs (4 floats each)
     std::vector<double> table_f64;     // TABLE entries as f64 (2 doubles each)
 };

@@ -1703,8 +1703,9 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
     std::vector<char> dig(np, 0);
     std::vector<DgPass> dgp(np);
     bool any_dig = false;
-    // (QGPU_PAIR2_TC selects the earlier tensor-core pair kernels instead)
-    if (!pre_resident && h->active == nullptr && dg_supported(h) && !pair2_tc_enabled()) {
+    // (QGPU_PAIR2_TC selects the earlier tensor-core pair kernels instead; a bound that Custom gates
+    // may have raised by more than 16 would cost the digits more than four of their 54 bits)
+    if (!pre_resident && h->active == nullptr && dg_supported(h) && !pair2_tc_enabled() && plan.growth <= 16.0) {
         static const int min_run = std::max(1, env_int("QGPU_DIGITS_MIN_RUN", 6));
         size_t i = 0;
         while (i < np) {
@@ -1810,7 +1811,7 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
     std::vector<LaunchItem> items;
     items.reserve(np + 8);
     int cur = pre_resident ? LAY_RES : LAY_PLAIN;
-    double bound = h->norm_bound;
+    double bound = h->norm_bound * plan.growth;
     int run_sx = dg::SX_UNIT;
     bool first_arith = true;
     for (size_t pi = 0; pi < np; ++pi) {
@@ -1887,7 +1888,11 @@ static int run_plan(qgpu_handle* h, const Plan& plan, bool sync = true, bool pre
         cv.sx = run_sx;
         items.push_back(cv);
     }
-    if (!pre_resident && h->active == nullptr) h->norm_bound = bound;
+    if (!pre_resident && h->active == nullptr) {
+        h->norm_bound = bound;
+        // (a bound that is only possible is looked up by the next call that needs one)
+        if (!(plan.growth <= 1.001)) h->norm_valid = false;
+    }
 
     const size_t nlaunch = items.size();
     std::vector<std::string> prof_names;
@@ -2130,7 +2135,7 @@ extern "C" int qgpu_apply_program(qgpu_handle* h, const qgpu_op* ops, size_t n_o
         size_t taken = 0;
         if (!gates.empty() && ops[at[0]].kind != QGPU_GATE_CUSTOM) {
             double bound = bound_before;
-            if (!(bound >= 0.0)) {
+            if (!(bound >= 0.0 && bound < 1e100)) {
                 double2 r;
                 int st = reduce_state(h, 0, &r);
                 if (st != QGPU_OK) return st;
@@ -2160,10 +2165,10 @@ extern "C" int qgpu_apply_program(qgpu_handle* h, const qgpu_op* ops, size_t n_o
     if (st != QGPU_OK) return st;
     // Fast mode carries f64 values as float pairs, which share the float32 exponent range: a
     // program whose Custom gates could grow the register's amplitudes past 2^100 (the running
-    // product of their effective maps' Frobenius norms times the register's bound) runs with
+    // product of their effective maps' norms times the register's bound) runs with
     // native f64 arithmetic instead of overflowing.
-    if (h->precision == QGPU_C128 && h->mode == QGPU_MODE_FAST && !plan.customs.empty()) {
-        double running = 1.0, peak = 1.0;
+    if (h->precision == QGPU_C128 && h->mode == QGPU_MODE_FAST && (!plan.customs.empty() || plan.growth > 2.0)) {
+        double running = plan.growth, peak = plan.growth;
         for (const LocalGate& g : plan.customs) {
             running *= custom_growth(g);
             peak = std::max(peak, running);
