@@ -336,7 +336,7 @@ def run_batch_leg(args) -> None:
             torch.distributed.barrier()
 
     for pname, prec in (("c128", nat.QGPU_C128), ("c64", nat.QGPU_C64)):
-        B.run_batch(cs[:8], precision=prec)  # warm-up (module load, graph path)
+        B.run_batch(cs[:8], precision=prec)  # warm-up (module load)
         tuned = {}
 
         def runner(part, prec=prec):

@@ -540,9 +540,10 @@ bool dg_build_image(const std::complex<double> M[16][16], uint32_t* bimg, int32_
 
 bool dg_supported(const qgpu_handle* h) {
     // tuning knobs, read per call: QGPU_DIGITS=0 keeps the float-pair kernels; digit runs are
-    // used from QGPU_DIGITS_MIN_QUBITS qubits (default 24: below that wide float-pair passes are
-    // faster, 20 brickwork layers at 20 / 22 / 23 / 24 qubits: 1.39 / 3.93 / 7.98 / 14.8 ms against
-    // 2.38 / 4.37 / 9.79 / 10.2 ms in digits)
+    // used from QGPU_DIGITS_MIN_QUBITS qubits (default 24: below that the float-pair passes the
+    // planner takes instead, pair passes for the most part, are faster; calls with 20 brickwork layers
+    // at 20 / 21 / 22 / 23 / 24 qubits: 1.10 / 2.10 / 3.04 / 7.45 / 11.6 ms against 2.31 / 3.33 / 4.28 / 9.79 /
+    // 10.2 ms in digits; with a Fourier transform behind them 1.57 ... 8.72 / 13.7 against 2.81 ... 11.1 / 12.4)
     const char* e = std::getenv("QGPU_DIGITS");
     const char* m = std::getenv("QGPU_DIGITS_MIN_QUBITS");
     const int on = e ? std::atoi(e) : 1;

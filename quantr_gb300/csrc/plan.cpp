@@ -1652,7 +1652,7 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
         // qubits, ansatz layers (dense 2x2s) 6.29 / 5.3 ms, random columns (mostly pair blocks) 5.46 /
         // 5.62 ms; 20 qubits, 40 random columns 0.58 / 0.39 ms, 20 brickwork layers 0.95 / 0.98 ms.)
         const bool by_time = opt.policy == POL_FF && n >= opt.wide_large_qubits;
-        const double launch = 5e-6 * 152 * 1.9e9 / std::ldexp(1.0, n);
+        const double launch = 5e-6 * 152 * 1.9e9 / std::ldexp(1.0, n);  // (a GB300's SMs and clock)
         double tile_time = 0.0;
         auto step_ops = [](const DevStep& d, double dense) {
             const double part = std::ldexp(1.0, -std::min(popcount64(d.cm), 8));

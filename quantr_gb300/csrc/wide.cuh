@@ -13,7 +13,7 @@
 // Against register-tile passes (k_tile, k_pair2) a wide pass does the work of three to ten of
 // them per trip through HBM (complex64) and per launch (small registers). Bound: arithmetic and
 // issue, the FMA pipe at 42 to 56 % of its cycles (24 qubits, complex128) and 29 to 48 %
-// (complex64); DRAM at 13 to 28 %.
+// (complex64, 29 to 36 % where every round is a pair block); DRAM at 13 to 28 %.
 // Measured, tile against wide passes, time on the GPU: 17 qubits of complex128, 40 random columns
 // 352 / 107 us (47 / 6 launches); 16-qubit ansatz, 4 layers 320 / 110 us; complex64 at 24 qubits 3.56 /
 // 1.5 ms; complex64 at 30 qubits, 4 brickwork layers 53.2 / 43.0 ms.
