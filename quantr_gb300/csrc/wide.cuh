@@ -454,28 +454,19 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
     const bool third_kept = ff && s.type != ST_DENSE && s.type != ST_DENSE4;
     const bool given = s.given || (s.type == ST_DENSE4 && plan.pairs[ws.pair].given);
     const bool phase = s.type == ST_PHASE && !s.unit && __builtin_popcountll(s.cm) == 1;
-    double size = 0.0, exact = 0.0;  // sum of x^2 over the entries, and its rounding
-    auto square = [&](double x) {
-        const double sq = x * x, sum = size + sq, b = sum - size;
-        exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
-        size = sum;
-    };
-    for (size_t k = 0; k < e.size() && (whole || phase); ++k) {
-        square(e[k].real());
-        if (s.type != ST_REAL) square(e[k].imag());
-    }
-    // sum |e|^2 of a unitary d x d matrix is d (false for sizes that are not finite)
-    const double d = given ? size : s.type == ST_DENSE4 ? 4.0 : s.type == ST_PHASE ? 1.0 : 2.0;
-    const bool known = given ? size > 0.0 && size < HUGE_VAL : std::fabs(size - d) < 1e-12;
-    const double off = given ? 0.0 : (size - d) + exact;
-    double change = 0.0;  // sum of x'^2 - x^2 for the entries x' that are uploaded
+    // sums of x^2 over the entries, of its rounding, and of x'^2 - x^2 for the entries x' uploaded
+    double size = 0.0, exact = 0.0, change = 0.0;
     auto part = [&](double x, float* h, float* l, float* third) {
-        const double y = whole && known ? x - x * *drift : x;
+        const double y = whole ? x - x * *drift : x;
         *h = (float)y;
         *l = pair32 ? 0.0f : (float)(y - (double)*h);
         *third = (float)((y - (double)*h) - (double)*l);
+        if (!whole && !phase) return;
         const double kept = ((double)*h + (double)*l) + (third_kept ? (double)*third : 0.0);
         change += (kept - x) * (kept + x);
+        const double sq = x * x, sum = size + sq, b = sum - size;
+        exact += std::fma(x, x, -sq) + ((size - (sum - b)) + (sq - b));
+        size = sum;
     };
     auto term = [&](float h, float l, float third, bool mixed) {  // hi, -third, -hi, -lo
         const float s0 = mixed ? -1.0f : 1.0f;  // (the real lane of an imaginary part)
@@ -498,9 +489,12 @@ static std::vector<u64> wide_constants(const Plan& plan, const WideStep& ws, dou
             if (s.type != ST_REAL && !pair32) c.push_back(wide_pack(il, il));
         }
     }
+    // sum |e|^2 of a unitary d x d matrix is d (sizes that are not finite count for nothing)
+    const double d = given ? size : s.type == ST_DENSE4 ? 4.0 : s.type == ST_PHASE ? 1.0 : 2.0;
+    const double off = given ? 0.0 : (size - d) + exact;
+    const bool known = given ? size > 0.0 && size < HUGE_VAL : std::fabs(size - d) < 1e-12;
     if (whole && known) *drift += 0.5 * (off + change) / d;
-    if (phase && known)
-        *drift += 0.25 * (off + change) / d;  // (half the amplitudes)
+    if (phase && known) *drift += 0.25 * (off + change) / d;  // (half the amplitudes)
     if (c.size() & 1) c.push_back(0);  // 16-byte aligned
     return c;
 }
