@@ -1511,123 +1511,123 @@ int build_plan(const qgpu_op* ops, size_t n_ops, int n, const double* mats, size
     };
     auto is_sw = [&](size_t i) { return block_at[i] < 0 && steps[i].s.type == ST_SWAP; };
     auto emit_tiles = [&](size_t begin, size_t end) {
-    for (size_t i = begin; i < end; ++i) {
-        if (block_at[i] >= 0) {
-            flush();
-            Pass p;
-            p.custom = block_at[i];
-            plan->passes.push_back(p);
-            continue;
-        }
-        if (opt.xor_runs && (is_cx(i) || is_sw(i))) {
-            // longest run of controlled-X / swap steps forming one involution
-            uint64_t targets = 0, controls = 0, swapped = 0;
-            size_t j = i;
-            while (j < end && (is_cx(j) || is_sw(j))) {
-                if (is_sw(j)) {
-                    const uint64_t sb = (1ull << steps[j].need[0]) | (1ull << steps[j].need[1]);
-                    if (sb & (targets | controls | swapped)) break;
-                    swapped |= sb;
-                } else {
-                    const uint64_t tb = 1ull << steps[j].need[0], cm = steps[j].s.cm;
-                    if ((targets & tb) || (targets & cm) || (controls & tb) || (swapped & (tb | cm)))
-                        break;
-                    targets |= tb;
-                    controls |= cm;
-                }
-                ++j;
-            }
-            XorPerm xp;
-            bool fits = j - i >= 3;
-            for (size_t q = i; q < j && fits; ++q) {
-                if (is_sw(q)) {
-                    if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
-                    const int g = xp.nterms++;
-                    xp.grouped[g] = 2;
-                    xp.shift[g] = 0;
-                    xp.cm[g] = (1ull << steps[q].need[0]) | (1ull << steps[q].need[1]);
-                    xp.tbit[g] = 0;
-                    continue;
-                }
-                const int t = steps[q].need[0];
-                const uint64_t cm = steps[q].s.cm;
-                if (popcount64(cm) == 1) {
-                    const int c = __builtin_ctzll(cm);
-                    const int shift = c - t;
-                    int g = -1;
-                    for (int e = 0; e < xp.nterms; ++e)
-                        if (xp.grouped[e] && xp.shift[e] == shift) g = e;
-                    if (g < 0) {
-                        if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
-                        g = xp.nterms++;
-                        xp.grouped[g] = 1;
-                        xp.shift[g] = shift;
-                        xp.cm[g] = 0;
-                        xp.tbit[g] = 0;
-                    }
-                    xp.cm[g] |= cm;
-                    xp.tbit[g] |= 1ull << t;
-                } else {
-                    if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
-                    const int g = xp.nterms++;
-                    xp.grouped[g] = 0;
-                    xp.shift[g] = 0;
-                    xp.cm[g] = cm;
-                    xp.tbit[g] = 1ull << t;
-                }
-            }
-            if (fits) {
+        for (size_t i = begin; i < end; ++i) {
+            if (block_at[i] >= 0) {
                 flush();
                 Pass p;
-                p.xor_pass = true;
-                p.xp = xp;
-                double touched = 0.0;
-                for (size_t q = i; q < j; ++q)
-                    touched += is_sw(q) ? 0.5 : std::ldexp(1.0, -popcount64(steps[q].s.cm));
-                p.touched = std::min(1.0, touched);
+                p.custom = block_at[i];
                 plan->passes.push_back(p);
-                i = j - 1;
                 continue;
             }
-        }
-        const HStep& h = steps[i];
-        if (h.s.type == ST_DENSE4) {  // a pair block is a pass of its own (k_pair)
-            flush();
-            Pass p;
-            p.nbits = 2;
-            p.bits[0] = std::min(h.need[0], h.need[1]);
-            p.bits[1] = std::max(h.need[0], h.need[1]);
-            p.arith = true;
-            p.cost = 380;
-            p.touched = 1.0;
-            p.pair = (int)h.s.tab_off[0];
-            plan->passes.push_back(p);
-            continue;
-        }
-        std::vector<int> bits = cur_bits;
-        for (int q = 0; q < 2; ++q)
-            if (h.need[q] >= 0 && std::find(bits.begin(), bits.end(), h.need[q]) == bits.end())
-                bits.push_back(h.need[q]);
-        const int c = step_cost(h, opt.policy);
-        const bool arith = !h.unit;
-        const int new_cost = cur_cost + c + ((arith && !cur_arith) ? conv : 0);
-        const int width = (arith || cur_arith) ? std::min(max_bits, std::max(1, opt.max_arith_bits))
-                                               : max_bits;
-        const bool fits = (int)bits.size() <= width && (int)cur_steps.size() < MAX_STEPS &&
-                          (cur_steps.empty() || new_cost <= opt.budget);
-        if (!fits) {
-            flush();
-            bits.clear();
+            if (opt.xor_runs && (is_cx(i) || is_sw(i))) {
+                // longest run of controlled-X / swap steps forming one involution
+                uint64_t targets = 0, controls = 0, swapped = 0;
+                size_t j = i;
+                while (j < end && (is_cx(j) || is_sw(j))) {
+                    if (is_sw(j)) {
+                        const uint64_t sb = (1ull << steps[j].need[0]) | (1ull << steps[j].need[1]);
+                        if (sb & (targets | controls | swapped)) break;
+                        swapped |= sb;
+                    } else {
+                        const uint64_t tb = 1ull << steps[j].need[0], cm = steps[j].s.cm;
+                        if ((targets & tb) || (targets & cm) || (controls & tb) || (swapped & (tb | cm)))
+                            break;
+                        targets |= tb;
+                        controls |= cm;
+                    }
+                    ++j;
+                }
+                XorPerm xp;
+                bool fits = j - i >= 3;
+                for (size_t q = i; q < j && fits; ++q) {
+                    if (is_sw(q)) {
+                        if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
+                        const int g = xp.nterms++;
+                        xp.grouped[g] = 2;
+                        xp.shift[g] = 0;
+                        xp.cm[g] = (1ull << steps[q].need[0]) | (1ull << steps[q].need[1]);
+                        xp.tbit[g] = 0;
+                        continue;
+                    }
+                    const int t = steps[q].need[0];
+                    const uint64_t cm = steps[q].s.cm;
+                    if (popcount64(cm) == 1) {
+                        const int c = __builtin_ctzll(cm);
+                        const int shift = c - t;
+                        int g = -1;
+                        for (int e = 0; e < xp.nterms; ++e)
+                            if (xp.grouped[e] && xp.shift[e] == shift) g = e;
+                        if (g < 0) {
+                            if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
+                            g = xp.nterms++;
+                            xp.grouped[g] = 1;
+                            xp.shift[g] = shift;
+                            xp.cm[g] = 0;
+                            xp.tbit[g] = 0;
+                        }
+                        xp.cm[g] |= cm;
+                        xp.tbit[g] |= 1ull << t;
+                    } else {
+                        if (xp.nterms == MAX_XOR_TERMS) { fits = false; break; }
+                        const int g = xp.nterms++;
+                        xp.grouped[g] = 0;
+                        xp.shift[g] = 0;
+                        xp.cm[g] = cm;
+                        xp.tbit[g] = 1ull << t;
+                    }
+                }
+                if (fits) {
+                    flush();
+                    Pass p;
+                    p.xor_pass = true;
+                    p.xp = xp;
+                    double touched = 0.0;
+                    for (size_t q = i; q < j; ++q)
+                        touched += is_sw(q) ? 0.5 : std::ldexp(1.0, -popcount64(steps[q].s.cm));
+                    p.touched = std::min(1.0, touched);
+                    plan->passes.push_back(p);
+                    i = j - 1;
+                    continue;
+                }
+            }
+            const HStep& h = steps[i];
+            if (h.s.type == ST_DENSE4) {  // a pair block is a pass of its own (k_pair)
+                flush();
+                Pass p;
+                p.nbits = 2;
+                p.bits[0] = std::min(h.need[0], h.need[1]);
+                p.bits[1] = std::max(h.need[0], h.need[1]);
+                p.arith = true;
+                p.cost = 380;
+                p.touched = 1.0;
+                p.pair = (int)h.s.tab_off[0];
+                plan->passes.push_back(p);
+                continue;
+            }
+            std::vector<int> bits = cur_bits;
             for (int q = 0; q < 2; ++q)
                 if (h.need[q] >= 0 && std::find(bits.begin(), bits.end(), h.need[q]) == bits.end())
                     bits.push_back(h.need[q]);
+            const int c = step_cost(h, opt.policy);
+            const bool arith = !h.unit;
+            const int new_cost = cur_cost + c + ((arith && !cur_arith) ? conv : 0);
+            const int width = (arith || cur_arith) ? std::min(max_bits, std::max(1, opt.max_arith_bits))
+                                                   : max_bits;
+            const bool fits = (int)bits.size() <= width && (int)cur_steps.size() < MAX_STEPS &&
+                              (cur_steps.empty() || new_cost <= opt.budget);
+            if (!fits) {
+                flush();
+                bits.clear();
+                for (int q = 0; q < 2; ++q)
+                    if (h.need[q] >= 0 && std::find(bits.begin(), bits.end(), h.need[q]) == bits.end())
+                        bits.push_back(h.need[q]);
+            }
+            cur_bits = bits;
+            cur_cost += c + ((arith && !cur_arith) ? conv : 0);
+            cur_arith = cur_arith || arith;
+            cur_steps.push_back(h);
         }
-        cur_bits = bits;
-        cur_cost += c + ((arith && !cur_arith) ? conv : 0);
-        cur_arith = cur_arith || arith;
-        cur_steps.push_back(h);
-    }
-    flush();
+        flush();
     };
     // Segments: Custom blocks, runs of pair blocks kept for the pair passes, runs of swaps (one
     // index permutation) and, between them, what wide passes may take.
