@@ -81,3 +81,30 @@ def test_exact_mode_after_growth_to_infinity(oracle):
     h.apply(prog.ops, prog.mats, prog.none)
     assert np.array_equal(h.download(), oracle.simulate(prog, reg, engine=oracle.DENSE), equal_nan=True)
     h.close()
+
+
+@pytest.mark.parametrize("growth", [3.0, 1e6])
+def test_growth_between_pair_passes(monkeypatch, oracle, growth):
+    """Kept apart from the pair blocks by Toffoli gates: digits up to a growth of 16, float pairs past it."""
+    monkeypatch.setenv("QGPU_DIGITS_MIN_QUBITS", "11")
+    n = 14
+    layers = W.brickwork_qft(n=n, layers=8, seed=6, qft=False)
+    b = ProgramBuilder(n)
+    for _ in range(2):
+        b.add("Toffoli", 4, (1, 9))
+        b.add_custom(4, [], np.eye(2, dtype=np.complex128) * growth ** 0.5, NONE)
+    b.add("Toffoli", 4, (0, 7))
+    grow = b.build()
+    prog = _joined(layers, grow, layers)
+    h = nat.Handle(n)
+    h.set_profiling(True)
+    h.apply(prog.ops, prog.mats, prog.none)
+    assert ("k_dg2" in h.profile()) == (growth <= 16.0)
+    _near(h.download(), oracle.simulate(prog, engine=oracle.DENSE_PAR))
+    h.close()
+
+
+def _joined(*programs):
+    """One program of several, of which only one has Custom gates (their tables stay where they are)."""
+    own = next(p for p in programs if p.mats.size)
+    return type(own)(own.n, np.concatenate([p.ops for p in programs]), own.mats, own.none)

@@ -107,3 +107,23 @@ def test_custom_gates_keep_their_scaling(oracle, kind):
     1.6e-11 and more, which is not taken for the rounding of library gates."""
     prof = _check(oracle, _chain(kind, 12, 20), nat.QGPU_C128)
     assert any(k.startswith("k_wide") for k in prof), prof
+
+
+@pytest.mark.parametrize("precision", [nat.QGPU_C128, nat.QGPU_C64])
+@pytest.mark.parametrize("n", [3, 4, 5, 6, 7, 10, 11, 12, 15])
+def test_transform_rows_around_the_lines(oracle, n, precision):
+    """Fourier transforms of a product state, between other layers, where their rows change between
+    wide and tile passes (11 qubits of complex128; two phase tables in a row of complex64)."""
+    b = ProgramBuilder(n)
+    for w in range(n):
+        b.add("Ry", w, (), param=0.3 + w)
+    for i in range(n):
+        b.add("H", i)
+        for k in range(2, n - i + 1):
+            b.add("CRk", i, (i + k - 1,), k=k)
+    for i in range(n // 2):
+        b.add("Swap", i, (n - 1 - i,))
+    for w in range(n):
+        b.add("Rx", w, (), param=0.2 * w - 1.0)
+        b.add("CNot", (w + 1) % n, (w,))
+    _check(oracle, b.build(), precision)
